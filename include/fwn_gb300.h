@@ -57,7 +57,8 @@ typedef enum fwn_status {
 
 /* Precision forms of the query. */
 enum {
-    FWN_PRECISION_MIXED = 0, /* FP32 traversal + far field, Kahan sum, FP64 for close triangles */
+    FWN_PRECISION_MIXED = 0, /* FP32 traversal + far field, Kahan sums, double-float or
+                                   FP64 for close ill-conditioned triangles */
     FWN_PRECISION_FP64 = 1   /* plain form: FP64 everywhere */
 };
 
@@ -99,19 +100,18 @@ typedef struct fwn_config {
     int32_t traversal;     /* default schedule, FWN_TRAVERSAL_*. Default AUTO */
     int32_t block_size;    /* query kernel block size (multiple of 32, <= 1024); 0 = tuned */
     int32_t sort_queries;  /* 1: sort queries along a Hilbert curve first (default), 0: input order */
-    float fp64_near_scale; /* FP64 near field if triangle is within scale*bbox_diagonal. 1e-3 */
+    float fp64_near_scale; /* near field beyond FP32 if triangle is within scale*bbox_diagonal. 1e-3 */
     float fp64_cond;       /* ... and its FP32 evaluation is ill-conditioned: |a||b||c| >
                               fp64_cond * |(det, D)|, or det is within rounding of 0 with D <= 0.
                               0 = every triangle within the distance. Default 4 */
     int32_t tuning;        /* warp-schedule variant (set by fwn_autotune): queries per lane and
                               register cap. 1: 1 query per lane, 72 registers; 2: 1, no cap;
-                              3: 1, 64 registers; 4: 2 queries per lane, 64 registers; 5: 2, 80;
-                              6: as 4 with both query slots' Taylor terms in paired f32x2
-                              arithmetic (same results bit for bit); 7: as 6 reading the node
+                              3: 1, 64 registers; 4 and 6: 2 queries per lane, 64 registers;
+                              5: 2, 80 (same results bit for bit); 7: as 6 reading the node
                               records from a structure-of-arrays copy (eight float4 arrays,
                               128 B more per node) that a build with tuning 7 keeps: the layout
                               comparison, one mesh's point queries only (grids and forests run 6).
-                              0 (default): 4 for batches that fill the GPU, else 3 */
+                              0 (default): 6 for batches that fill the GPU, else 3 */
     int32_t builder;       /* FWN_BUILDER_*. Default FWN_BUILDER_LBVH */
     int32_t reserved[5];
 } fwn_config;

@@ -200,6 +200,7 @@ struct Engine {
     fwn_config cfg;
     int64_t nv = 0, nf = 0, nmeshes = 0;
     int64_t num_nodes = 0, num_leaves = 0;
+    int leaf_cap = 1;              // triangles in the largest leaf, at most (sizes the walks' buffers)
     NodeF32* nodes32 = nullptr;
     NodeF64* nodes64 = nullptr;
     float4* soa = nullptr;         // the FP32 records as 8 float4 arrays (tuning 7 builds only)

@@ -2016,6 +2016,7 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     e.nf = nf;
     e.nmeshes = nmeshes;
     const int K = e.cfg.leaf_size;
+    e.leaf_cap = K;
     NvtxRange trace_build("fwn build");
 
     cudaEvent_t ev0, ev1;

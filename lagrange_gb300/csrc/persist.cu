@@ -12,6 +12,7 @@
 // A load checks the magic, version, sizes and checksum before it touches the device, then every
 // node's links and triangle range and every mesh's root range, so that a file the walk would
 // read out of bounds with is refused instead of queried.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -73,16 +74,20 @@ void read_exact(FILE* f, void* p, size_t n, Fnv* sum) {
 }
 
 // The walk follows skip links forward and reads a leaf's triangles [tri_begin, tri_begin +
-// tri_count); a mesh's walk runs over [root, end).
+// tri_count); a mesh's walk runs over [root, end). Returns the triangles of the largest leaf, at
+// least 1 (the walks' buffers are sized by it).
 template <class Node>
-void check_nodes(const std::vector<Node>& nodes, int64_t nf) {
+int check_nodes(const std::vector<Node>& nodes, int64_t nf) {
     const int64_t E = (int64_t)nodes.size();
+    int cap = 1;
     for (int64_t i = 0; i < E; ++i) {
         const Node& n = nodes[(size_t)i];
         if (n.skip <= i || n.skip > E || n.tri_count < 0 || n.tri_count > 16 || n.tri_begin < 0 ||
             (int64_t)n.tri_begin + n.tri_count > nf)
             throw Error(FWN_INVALID_ARG, "engine file holds an inconsistent node " + std::to_string(i));
+        cap = std::max(cap, (int)n.tri_count);
     }
+    return cap;
 }
 
 }  // namespace
@@ -205,8 +210,9 @@ extern "C" FWN_API fwn_status fwn_load(const char* path, fwn_handle* out) {
         read_exact(f.f, tris.data(), tris.size() * sizeof(TriF32), &sum);
         read_exact(f.f, sorted.data(), sorted.size() * sizeof(int), &sum);
         if (sum.h != hd.checksum) throw Error(FWN_INVALID_ARG, "engine file is corrupt (checksum)");
-        if (hd.has32) check_nodes(n32, nf);
-        if (hd.has64) check_nodes(n64, nf);
+        int leaf_cap = 1;
+        if (hd.has32) leaf_cap = std::max(leaf_cap, check_nodes(n32, nf));
+        if (hd.has64) leaf_cap = std::max(leaf_cap, check_nodes(n64, nf));
         for (const MeshInfo& m : meshes)
             if (!(m.root == -1 && m.end == -1) && !(m.root >= 0 && m.root < m.end && m.end <= E))
                 throw Error(FWN_INVALID_ARG, "engine file holds an inconsistent mesh root");
@@ -220,6 +226,7 @@ extern "C" FWN_API fwn_status fwn_load(const char* path, fwn_handle* out) {
         e->nmeshes = M;
         e->num_nodes = E;
         e->num_leaves = hd.num_leaves;
+        e->leaf_cap = leaf_cap;
         e->nodes32 = to_device(n32);
         e->nodes64 = to_device(n64);
         e->tris = to_device(tris);
