@@ -162,6 +162,34 @@ cudaStream_t host_stream(int k = 0) {
     return t.s[dev][k];
 }
 
+// Pinned host memory that a small fwn_query_host call stages its points and results in and its kernel
+// reads and writes directly: per (host thread, device), made on first use and kept, like the
+// streams, for the thread's lifetime (68 KB).
+constexpr int64_t kStagePoints = 4096;
+
+struct HostStage {
+    float points[3 * kStagePoints];
+    float omega[kStagePoints];
+    uint8_t inside[kStagePoints];
+    unsigned status;
+};
+
+HostStage* host_stage() {
+    struct Stages {
+        HostStage* s[kMaxDevices] = {};
+        ~Stages() {
+            for (HostStage* x : s)
+                if (x) cudaFreeHost(x);
+        }
+    };
+    thread_local Stages t;
+    int dev = 0;
+    FWN_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) throw Error(FWN_INTERNAL, "device ordinal out of range");
+    if (!t.s[dev]) FWN_CUDA_CHECK(cudaMallocHost(&t.s[dev], sizeof(HostStage)));
+    return t.s[dev];
+}
+
 Engine* engine_of(fwn_handle h) {
     if (!h) throw Error(FWN_NOT_BUILT, "null handle (default-constructed or moved-from engine)");
     return reinterpret_cast<Engine*>(h);
@@ -351,6 +379,20 @@ FWN_API fwn_status fwn_query_host(fwn_handle h, const float* points, int64_t n, 
         if (n == 0) return;
         QueryArgs a = resolve_query_args(*e, nullptr);
         const cudaStream_t st = host_stream();
+        if (n <= kStagePoints) {  // no copies, no scratch: the walk works on staged host memory
+            HostStage* h = host_stage();
+            std::memcpy(h->points, points, n * 3 * sizeof(float));
+            h->status = 0;
+            if (query_mesh_single(*e, 0, a, h->points, n, omega ? h->omega : nullptr,
+                                  inside ? h->inside : nullptr, &h->status, st)) {
+                FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+                if (h->status & ST_BAD_LINK)
+                    throw Error(FWN_INTERNAL, "traversal met a non-advancing skip link");
+                if (omega) std::memcpy(omega, h->omega, n * sizeof(float));
+                if (inside) std::memcpy(inside, h->inside, n);
+                return;
+            }
+        }
         Scratch dq(n * 3 * sizeof(float), st);
         Scratch dw(omega ? n * sizeof(float) : 0, st);
         Scratch di(inside ? n * sizeof(uint8_t) : 0, st);

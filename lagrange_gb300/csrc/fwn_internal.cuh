@@ -250,6 +250,11 @@ struct QueryArgs {
 void query_mesh(const Engine& e, int mesh, const QueryArgs& a, const float* d_points, int64_t n,
                 float* d_omega, uint8_t* d_inside, double* d_omega64, fwn_query_stats* stats,
                 cudaStream_t stream, bool check = false);
+// The same in one launch of one warp per query, without scratch, reading and writing any memory that
+// the device can address: false (and nothing done) where n is too large for it or the arguments ask
+// for another form. `status` (zeroed by the caller) gets the device status bits. Async.
+bool query_mesh_single(const Engine& e, int mesh, const QueryArgs& a, const float* points, int64_t n,
+                       float* omega, uint8_t* inside, unsigned* status, cudaStream_t stream);
 // Regular voxel-centre grid of mesh `mesh` (no point array); outputs indexed i + nx (j + ny k).
 void query_grid(const Engine& e, int mesh, const QueryArgs& a, const float origin[3],
                 const float spacing[3], const int64_t dims[3], float* d_omega, uint8_t* d_inside,
