@@ -62,11 +62,12 @@ enum {
     FWN_PRECISION_FP64 = 1   /* plain form: FP64 everywhere */
 };
 
-/* Traversal schedules. AUTO is the warp schedule for the mixed form and the thread schedule
- * (the plain form) for the FP64 form; the FP64 form runs on the warp schedule when WARP is asked
- * for explicitly (same cursor and leaf pairs, FP64 arithmetic, same sums as the thread form). */
+/* Traversal schedules. AUTO picks by form and batch: the mixed form's warp schedule, or for batches
+ * too small to fill the GPU one warp per query (the same bits); one warp per query for the FP64
+ * form. The FP64 form runs on the thread schedule (the plain form) or the warp schedule when THREAD
+ * or WARP is asked for explicitly (FP64 arithmetic throughout; the schedules agree to 1e-12 in w). */
 enum {
-    FWN_TRAVERSAL_AUTO = 0,   /* mixed: autotuned warp schedule; FP64: thread schedule */
+    FWN_TRAVERSAL_AUTO = 0,   /* mixed: warp schedule; FP64 and small batches: a warp per query */
     FWN_TRAVERSAL_THREAD = 1, /* one thread per query, stackless skip-link walk */
     FWN_TRAVERSAL_WARP = 2    /* warp-shared cursor over 32 queries, leaf triangles in smem */
 };
