@@ -1513,23 +1513,110 @@ __global__ void k_leaf_sort(int nl, const int* __restrict__ leaves, const int* _
 
 // The internal nodes of one level of a split tree, or of one height of the LBVH
 // (nodes[0 .. count)): each combines its two children, whose records the leaf pass or an
-// earlier (deeper, or lower) list wrote.
-__global__ void __launch_bounds__(128, 4) k_refit_level(int count, const int* __restrict__ nodes,
+// earlier (deeper, or lower) list wrote. A combine is some 270 FP64 instructions, and an SM issues
+// one FP64 warp instruction in 16 cycles, so the few warps of a small level are spread: one warp
+// per block (four to a block cost 10 us in the smallest levels), and levels that do not fill the
+// GPU (kLaneLevel) take the lane form below, 5 us. A level of 130,000 nodes takes 53 us: FP64 issue.
+__device__ __forceinline__ bool refit_children(const int* __restrict__ left,
+                                               const int* __restrict__ right,
+                                               const int* __restrict__ pos, int p, int& l, int& r,
+                                               unsigned* __restrict__ status) {
+    l = left[p];
+    r = right[p];
+    if (l >= 0 && r >= 0) {
+        l = pos[l];
+        r = pos[r];
+    }
+    if (l < 0 || r < 0) {
+        atomicOr(status, ST_REFIT_ORPHAN);
+        return false;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(32) k_refit_level(int count, const int* __restrict__ nodes,
                               const int* __restrict__ left, const int* __restrict__ right,
                               const int* __restrict__ pos, StageRec* __restrict__ stage,
                               unsigned* __restrict__ status) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int p = nodes[k];
-    const int l = left[p], r = right[p];
-    if (l < 0 || r < 0 || pos[l] < 0 || pos[r] < 0) {
-        atomicOr(status, ST_REFIT_ORPHAN);
-        return;
-    }
+    int l, r;
+    if (!refit_children(left, right, pos, p, l, r, status)) return;
     StageRec R;
-    combine_moments(&stage[pos[l]], &stage[pos[r]], R);
+    combine_moments(&stage[l], &stage[r], R);
     store_rec(&stage[pos[p]], R);
 }
+
+// The same combine (every operation of combine_moments, with the same bits) by four lanes: lane
+// i < 3 takes the i-th component of P and N and the i-th rows of M1 and M2.
+__global__ void __launch_bounds__(32) k_refit_level_lanes(
+    int count, const int* __restrict__ nodes, const int* __restrict__ left,
+    const int* __restrict__ right, const int* __restrict__ pos, StageRec* __restrict__ stage,
+    unsigned* __restrict__ status) {
+    const int k = (blockIdx.x * 32 + threadIdx.x) >> 2, i = threadIdx.x & 3;
+    int p = -1, l = -1, r = -1;
+    if (k < count && i < 3) {
+        p = nodes[k];
+        if (!refit_children(left, right, pos, p, l, r, status)) p = -1;
+    }
+    const bool on = p >= 0;
+    const double* ra = reinterpret_cast<const double*>(stage + (on ? l : 0));
+    const double* rb = reinterpret_cast<const double*>(stage + (on ? r : 0));
+    double Na = 0.0, Nb = 0.0, M1a[3], M1b[3], M2a[6], M2b[6];
+    double A = 0.0, P = 0.0, ea = 0.0, eb = 0.0;
+    if (on) {
+        const double Aa = ra[3], Ab = rb[3], Pa = ra[i], Pb = rb[i];
+        Na = ra[4 + i];
+        Nb = rb[4 + i];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            M1a[j] = ra[7 + 3 * i + j];
+            M1b[j] = rb[7 + 3 * i + j];
+            const double2 x = ld_rec2(ra + 16 + 6 * i + 2 * j), y = ld_rec2(rb + 16 + 6 * i + 2 * j);
+            M2a[2 * j] = x.x;
+            M2a[2 * j + 1] = x.y;
+            M2b[2 * j] = y.x;
+            M2b[2 * j + 1] = y.y;
+        }
+        A = Aa + Ab;
+        const double pe = A > 0.0 ? fmad(Aa, Pa, Ab * Pb) / A : (Pa + Pb) * 0.5;
+        P = f2d(d2f(pe));
+        ea = Pa - P;
+        eb = Pb - P;
+    }
+    double va[3], vb[3];
+    const int lane0 = threadIdx.x & 28;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        va[j] = __shfl_sync(0xffffffffu, ea, lane0 + j);
+        vb[j] = __shfl_sync(0xffffffffu, eb, lane0 + j);
+    }
+    if (!on) return;
+    double* R = reinterpret_cast<double*>(stage + pos[p]);
+    R[i] = P;
+    R[4 + i] = Na + Nb;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        R[7 + 3 * i + j] = fmad(Na, va[j], M1a[j]) + fmad(Nb, vb[j], M1b[j]);
+    const int SJ[6] = {0, 1, 2, 0, 0, 1};
+    const int SK[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int j = SJ[q], m = SK[q];
+        const double ta = fmad(Na, va[j] * va[m], fmad(M1a[m], va[j], fmad(M1a[j], va[m], M2a[q])));
+        const double tb = fmad(Nb, vb[j] * vb[m], fmad(M1b[m], vb[j], fmad(M1b[j], vb[m], M2b[q])));
+        R[16 + 6 * i + q] = ta + tb;
+    }
+    if (i == 0) {
+        R[3] = A;
+        R[34] = 0.0;  // r: exact radius about P, k_node_radius after the refit
+        R[35] = 0.0;  // pad
+    }
+}
+// At 8,192 nodes the two forms meet: the lane form takes 8 us there; the thread form 13 us at 16,000,
+// where the lane form's repeated address work and its 1.4 times as many FP64 instructions show.
+constexpr int kLaneLevel = 8192;
 
 // LBVH: the height of every emitted internal node (a leaf is 0, a node one more than its taller
 // child), by an integer ascent from the emitted leaves (the second child to arrive continues);
@@ -2362,8 +2449,12 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             for (int h = 0; h < kMaxHeight; ++h) off[h + 1] = off[h] + h_hist[h];
             for (int t = 0; t < kMaxHeight; ++t) {
                 const int h = split ? kMaxHeight - 1 - t : t;
-                if (h_hist[h] > 0)
-                    k_refit_level<<<grid_for(h_hist[h], 128), 128, 0, st>>>(
+                if (h_hist[h] == 0) continue;
+                if (h_hist[h] <= kLaneLevel)
+                    k_refit_level_lanes<<<grid_for(h_hist[h], 8), 32, 0, st>>>(
+                        h_hist[h], order + off[h], left, right, pos, stage, status);
+                else
+                    k_refit_level<<<grid_for(h_hist[h], 32), 32, 0, st>>>(
                         h_hist[h], order + off[h], left, right, pos, stage, status);
             }
         }

@@ -1,0 +1,61 @@
+"""GPU tests of the build at sizes where its kernels change form: levels of a few nodes and of
+thousands (the refit's lane and thread forms), triangles without area, and meshes around the
+split builders' whole-block segments. Against the CPU restatement of the build: topology, order,
+centres and radii bit for bit; FP64 moments to 1e-12 of their largest (tests/test_gpu_parity.py)."""
+import numpy as np
+import pytest
+
+import lagrange_gb300 as fwn
+from lagrange_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+ALL = fwn.RECORDS_F32 | fwn.RECORDS_F64 | fwn.RECORDS_MOMENTS
+
+
+@pytest.fixture(scope="module")
+def torch():
+    t = pytest.importorskip("torch")
+    if not t.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    return t
+
+
+def _compare(oracle_mod, V, F, leaf, builder):
+    got = fwn.FastWindingNumber(V, F, records=ALL, leaf_size=leaf, builder=builder)
+    m, got = got.export_moments(), got.export_tree()
+    ref = oracle_mod.LbvhTree(V, F, leaf_size=leaf, builder=builder).export()
+    for k in ("skip", "tri_begin", "tri_count", "sorted_tri", "mesh_root"):
+        np.testing.assert_array_equal(got[k], ref[k], err_msg=k)
+    np.testing.assert_array_equal(got["center_radius"], ref["center_radius"])
+    scale = np.max(np.abs(ref["moments"]), axis=0) + 1e-300
+    assert np.max(np.abs(m - ref["moments"]) / scale) <= 1e-12
+
+
+@pytest.mark.parametrize("builder", [fwn.BUILDER_LBVH, fwn.BUILDER_SPLIT, fwn.BUILDER_BINNED])
+@pytest.mark.parametrize("n", [1, 2, 3, 9, 17, 33, 257, 1024, 1025, 2049, 5000])
+def test_small_levels(torch, oracle_mod, builder, n):
+    """n random triangles, a third of them without area (the centre falls back to plain means)."""
+    rng = np.random.default_rng(n)
+    V = rng.normal(size=(3 * n, 3)).astype(np.float32)
+    V[1::9] = V[0::9][:len(V[1::9])]
+    V[2::9] = V[0::9][:len(V[2::9])]
+    _compare(oracle_mod, V, np.arange(3 * n, dtype=np.int32).reshape(-1, 3), 1, builder)
+
+
+@pytest.mark.parametrize("builder", [fwn.BUILDER_LBVH, fwn.BUILDER_SPLIT, fwn.BUILDER_BINNED])
+def test_large_levels(torch, oracle_mod, builder):
+    """51,200 triangles, one per leaf: levels on both sides of the refit's change of form."""
+    wl = W.displaced_icosphere_workload(nu=50, n_queries=1)
+    assert len(wl.F) > 4 * 8192
+    _compare(oracle_mod, wl.V, wl.F, 1, builder)
+
+
+@pytest.mark.parametrize("builder", [fwn.BUILDER_SPLIT, fwn.BUILDER_BINNED])
+@pytest.mark.parametrize("n", [1500, 6000])
+def test_coincident_centroids(torch, oracle_mod, builder, n):
+    """Every centroid in one place (splits by position), and one far away (splits of one)."""
+    rng = np.random.default_rng(7)
+    T = rng.integers(-4, 5, size=(n, 3, 3)).astype(np.float32)
+    T[:, 2] = -T[:, 0] - T[:, 1]  # centroids at the origin, exactly
+    T[0] += 1000
+    _compare(oracle_mod, T.reshape(-1, 3), np.arange(3 * n, dtype=np.int32).reshape(-1, 3), 4, builder)
