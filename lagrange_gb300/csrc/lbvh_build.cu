@@ -23,7 +23,9 @@
 // individually rounded, in the order written, so the CPU restatement of the same build
 // (oracle/fwn_oracle.c, compiled with -ffp-contract=off) reproduces keys, topology, centres and
 // radii bit for bit.
+#include <algorithm>
 #include <cmath>
+#include <numeric>
 #include <utility>
 #include <vector>
 
@@ -382,12 +384,30 @@ __device__ __forceinline__ int split_bin(float x, float lo, float ext) {
 }
 
 struct SplitSlots {
-    int* perm;  // triangle id per slot
-    float* cx;  // its centroid
-    float* cy;
-    float* cz;
-    int* seg;   // active segment of the slot at this level (-1: in a leaf)
+    float4* tri;  // the slot's triangle: centroid, and its id as bits (one 16 B access)
+    int* seg;     // active segment of the slot at this level (-1: in a leaf)
 };
+
+// The level loop's state on the device: the host launches a level before it has seen the one before
+// (its grids come from bounds), so the kernels read their level's segment count here.
+constexpr int kMaxLevels = kSpatialLevels + 66;
+constexpr int kMaxHeight = 4 * 64 + 64;  // key bits + index bits bound the depth
+struct BuildState {
+    unsigned status;
+    int small_len;             // small segments listed
+    int finish_nodes;          // nodes made by k_split_finish
+    int done;                  // blocks of the running k_split_flags that are through
+    int2 level[kMaxLevels + 1];  // active segments; nodes made before
+    int internal[kMaxHeight];  // internal nodes by depth (split) or height (LBVH)
+};
+struct LevelBound {
+    int level, cap, segments;  // at most: nodes in all, active segments of a level
+};
+// The level's active segments: 0 (and ST_BUILD_BOUND, from k_split_children) past a bound.
+__device__ __forceinline__ int level_segments(const BuildState* st, LevelBound lb) {
+    const int2 v = st->level[lb.level];
+    return v.x > lb.segments || v.y + 2 * v.x > lb.cap ? 0 : v.x;
+}
 
 // A level of at most kBoxCopyKeys segments accumulates its boxes in kBoxCopies copies (block b
 // adds to copy b % kBoxCopies, copies kBoxCopyKeys boxes apart), merged by k_split_decide: at the
@@ -514,10 +534,7 @@ __global__ void k_split_init(const float* __restrict__ V, const int32_t* __restr
             for (int a = 0; a < 3; ++a) c[a] = ((v[0][a] + v[1][a]) + v[2][a]) / 3.0f;
         }
         key = mesh_seg[m];
-        out.perm[t] = (int)t;
-        out.cx[t] = c[0];
-        out.cy[t] = c[1];
-        out.cz[t] = c[2];
+        out.tri[t] = make_float4(c[0], c[1], c[2], __int_as_float((int)t));
         out.seg[t] = key;
         if (key == -1) final_perm[t] = (int)t;  // the whole mesh is one leaf (-2: a small root)
         keys[t] = (uint64_t)m << MORTON_BITS;
@@ -553,11 +570,15 @@ __device__ __forceinline__ void split_decide(const unsigned* __restrict__ box, i
     spatial_out = (!by_position && ext > 0.f && split > lo[axis]) ? 1 : 0;
 }
 
-__global__ void k_split_decide(int nact, bool by_position, const unsigned* __restrict__ box,
-                               int* __restrict__ axis_of, float* __restrict__ split_of,
-                               int* __restrict__ spatial_of, float* __restrict__ seg_box) {
+// (for the binned planes; the midpoint builder's k_split_flags decides for itself)
+__global__ void k_split_decide(const BuildState* __restrict__ bst, LevelBound lb,
+                               const unsigned* __restrict__ box, int* __restrict__ axis_of,
+                               float* __restrict__ split_of, int* __restrict__ spatial_of,
+                               float* __restrict__ seg_box) {
     const int sg = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nact = level_segments(bst, lb);
     if (sg >= nact) return;
+    const bool by_position = lb.level >= kSpatialLevels;
     unsigned b[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) b[a] = box[6 * sg + a];
@@ -576,8 +597,10 @@ __global__ void k_split_decide(int nact, bool by_position, const unsigned* __res
     for (int a = 0; a < 6; ++a) seg_box[6 * sg + a] = dec_float(b[a]);  // lo[3], hi[3]
 }
 
-__global__ void k_split_bins_init(int nwords, unsigned* __restrict__ bins) {
+__global__ void k_split_bins_init(const BuildState* __restrict__ bst, LevelBound lb,
+                                  unsigned* __restrict__ bins) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nwords = level_segments(bst, lb) * kSegBinWords;
     if (i >= nwords) return;
     const int w = i % kBinWords;
     bins[i] = w == 0 ? 0u : (w < 4 ? 0xffffffffu : 0u);  // count, lo (min of nothing), hi
@@ -586,10 +609,11 @@ __global__ void k_split_bins_init(int nwords, unsigned* __restrict__ bins) {
 // Per-segment bins of one level: a block takes kBinChunk consecutive slots, which meet at most
 // three of the level's segments (each holds more than kFinishSlots), accumulates their bins in
 // shared memory, then adds the non-empty ones to the segments' global bins.
-__global__ void __launch_bounds__(256) k_split_bins(int64_t n, SplitSlots cur,
+__global__ void __launch_bounds__(256) k_split_bins(int64_t n, BuildState* __restrict__ bst,
+                                                    LevelBound lb, SplitSlots cur,
                                                     const float* __restrict__ seg_box,
-                                                    unsigned* __restrict__ bins,
-                                                    unsigned* __restrict__ status) {
+                                                    unsigned* __restrict__ bins) {
+    if (level_segments(bst, lb) == 0) return;
     constexpr int kLocal = 4;
     __shared__ int tab[kLocal];
     __shared__ int ntab;
@@ -611,7 +635,7 @@ __global__ void __launch_bounds__(256) k_split_bins(int64_t n, SplitSlots cur,
         if (sg >= 0 && (i == c0 || cur.seg[i - 1] != sg)) {
             const int k = atomicAdd(&ntab, 1);
             if (k < kLocal) tab[k] = sg;
-            else atomicOr(status, ST_BUILD_BOUND);  // cannot happen: segments hold > 1024 slots
+            else atomicOr(&bst->status, ST_BUILD_BOUND);  // cannot happen: segments hold > 1024 slots
         }
     }
     __syncthreads();
@@ -626,9 +650,10 @@ __global__ void __launch_bounds__(256) k_split_bins(int64_t n, SplitSlots cur,
                 if (tab[k] == sg) slot = k;  // at most three segments meet a chunk
         float c[3] = {0.f, 0.f, 0.f};
         if (slot >= 0) {
-            c[0] = cur.cx[i];
-            c[1] = cur.cy[i];
-            c[2] = cur.cz[i];
+            const float4 x = cur.tri[i];
+            c[0] = x.x;
+            c[1] = x.y;
+            c[2] = x.z;
         }
         const unsigned ec[3] = {enc_float(c[0]), enc_float(c[1]), enc_float(c[2])};
 #pragma unroll
@@ -737,12 +762,13 @@ __device__ __forceinline__ void bin_scan_down(unsigned& n, float (&lo)[3], float
     }
 }
 
-__global__ void k_split_choose(int nact, const float* __restrict__ seg_box,
+__global__ void k_split_choose(const BuildState* __restrict__ bst, LevelBound lb,
+                               const float* __restrict__ seg_box,
                                const unsigned* __restrict__ bins, int* __restrict__ axis_of,
                                int* __restrict__ bin_of, int* __restrict__ spatial_of) {
     const int sg = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (sg >= nact) return;  // warp-uniform
+    if (sg >= level_segments(bst, lb)) return;  // warp-uniform
     const unsigned* sgb = bins + (int64_t)sg * kSegBinWords;
     double best = INFINITY;
     int best_a = 3, best_j = kSplitBins;
@@ -805,54 +831,185 @@ __global__ void k_split_choose(int nact, const float* __restrict__ seg_box,
     }
 }
 
-__global__ void k_split_flags(int64_t n, SplitSlots cur, const int* __restrict__ s_start,
-                              const int* __restrict__ s_end, const int* __restrict__ axis_of,
-                              const float* __restrict__ split_of,
-                              const int* __restrict__ spatial_of, const int* __restrict__ bin_of,
-                              const float* __restrict__ seg_box, int* __restrict__ flags) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    int f = 0;
-    if (i < n) {
-        const int sg = cur.seg[i];
-        if (sg >= 0) {
-            if (spatial_of[sg] == 2) {
-                const int a = axis_of[sg];
-                const float c = a == 0 ? cur.cx[i] : a == 1 ? cur.cy[i] : cur.cz[i];
-                const float lo = seg_box[6 * sg + a], ext = seg_box[6 * sg + 3 + a] - lo;
-                f = split_bin(c, lo, ext) <= bin_of[sg] ? 1 : 0;
-            } else if (spatial_of[sg]) {
-                const int a = axis_of[sg];
-                const float c = a == 0 ? cur.cx[i] : a == 1 ? cur.cy[i] : cur.cz[i];
-                f = c < split_of[sg] ? 1 : 0;
-            } else {
-                f = (i - s_start[sg]) < (s_end[sg] - s_start[sg]) / 2 ? 1 : 0;
-            }
-        }
-    }
-    flags[i] = f;  // flags[n] = 0: the scan's total entry
+// The left flags of a level, one bit per slot, with what turns a slot into its rank among all left
+// slots (left_rank): per 32 slots the count before them in their tile of kSplitTile slots, and per
+// tile the count before the tile (the grid's last block scans those). A tile meets at most two
+// active segments, those of its first and last slot (each holds more than kFinishSlots), so the
+// block decides their midpoint splits itself. Measured at 2 million slots: 14 us a level, most of
+// it latency (the state, the split, the slots, the last block); deciding, flags and a three-pass
+// scan of one int per slot took 32 us in five launches. With the records of 16 B that the scatter
+// moves (16 us; 19 as four arrays) and no round trip a level takes 41 us instead of 81.
+constexpr int kSplitTile = 1024;
+static_assert(kSplitTile <= kFinishSlots, "a tile meets at most two active segments");
+constexpr int kFlagThreads = 256;
+
+struct LeftRanks {
+    unsigned* bits;   // per 32 slots: left flags
+    int* in_tile;     // per 32 slots: left slots before them in their tile
+    int* tile;        // per tile: left slots before it
+};
+__device__ __forceinline__ int left_rank(const LeftRanks& r, int i) {
+    return r.tile[i / kSplitTile] + r.in_tile[i >> 5] +
+           __popc(r.bits[i >> 5] & ((1u << (i & 31)) - 1u));
 }
 
-// Children of every active segment (lf = exclusive scan of the left flags): the two nodes (at
-// depth level + 1), and for each child of more than kFinishSlots triangles a slot of the next
-// level (allocated with an atomic counter, its box cleared); a child of K < size <= kFinishSlots
-// triangles goes to the small list {start, end, node, depth} that k_split_finish completes.
-// child_next[2s + c] = the next level's slot, -2 for a small child or -1 for a leaf. The order
-// of segments in either list is immaterial: positions come from the node ranges alone.
-// counts[0] / counts[1]: the next level's segments / the small list's length.
-__global__ void k_split_children(int nact, int node_base, int level, int K,
+template <bool BINNED>
+__global__ void __launch_bounds__(kFlagThreads)
+k_split_flags(int64_t n, BuildState* __restrict__ bst, LevelBound lb, SplitSlots cur,
+              const int* __restrict__ s_start, const int* __restrict__ s_end,
+              const unsigned* __restrict__ box, const int* __restrict__ axis_of,
+              const float* __restrict__ split_of, const int* __restrict__ spatial_of,
+              const int* __restrict__ bin_of, const float* __restrict__ seg_box, LeftRanks ranks) {
+    constexpr int kRounds = kSplitTile / kFlagThreads, kWarps = kFlagThreads / 32;
+    __shared__ struct { int seg, axis, spatial; float split; } sp[2];
+    __shared__ int wc[kSplitTile / 32];
+    __shared__ bool last;
+    const int nact = level_segments(bst, lb);
+    if (nact == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * kSplitTile;
+    int seg[kRounds];  // all loads in flight before the split is known
+    float4 c[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int64_t i = base + r * kFlagThreads + threadIdx.x;
+        seg[r] = i < n ? cur.seg[i] : -1;
+        c[r] = i < n ? cur.tri[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (!BINNED && warp < 2) {
+        const int64_t at = warp == 0 ? base : min(base + kSplitTile, n) - 1;
+        const int sg = at >= 0 && at < n ? cur.seg[at] : -1;
+        if (sg >= 0) {
+            const unsigned* b = box + 6 * sg;
+            if (nact <= kBoxCopyKeys) b += (lane % kBoxCopies) * kBoxCopyStride;  // merge the copies
+            unsigned m[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a)
+                m[a] = a < 3 ? __reduce_min_sync(0xffffffffu, b[a]) : __reduce_max_sync(0xffffffffu, b[a]);
+            if (lane == 0)
+                split_decide(m, 1, lb.level >= kSpatialLevels, sp[warp].axis, sp[warp].split,
+                             sp[warp].spatial);
+        }
+        if (lane == 0) sp[warp].seg = sg;
+    }
+    if (!BINNED) __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int64_t i = base + r * kFlagThreads + threadIdx.x;
+        const int sg = seg[r];
+        bool f = false;
+        if (sg >= 0) {
+            int a, spatial;
+            float split;
+            if (BINNED) {
+                spatial = spatial_of[sg];
+                a = axis_of[sg];
+                split = split_of[sg];
+            } else {
+                const int k = sg == sp[0].seg ? 0 : 1;
+                spatial = sp[k].spatial;
+                a = sp[k].axis;
+                split = sp[k].split;
+            }
+            if (spatial) {
+                const float x = a == 0 ? c[r].x : a == 1 ? c[r].y : c[r].z;
+                if (BINNED && spatial == 2) {
+                    const float lo = seg_box[6 * sg + a], ext = seg_box[6 * sg + 3 + a] - lo;
+                    f = split_bin(x, lo, ext) <= bin_of[sg];
+                } else {
+                    f = x < split;
+                }
+            } else {
+                f = (i - s_start[sg]) < (s_end[sg] - s_start[sg]) / 2;
+            }
+        }
+        const unsigned w = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) {
+            wc[r * kWarps + warp] = __popc(w);
+            const int64_t g = (base >> 5) + r * kWarps + warp;
+            if (g <= (n >> 5)) ranks.bits[g] = w;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int own = wc[lane];
+        int x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const int64_t g = (base >> 5) + lane;
+        if (g <= (n >> 5)) ranks.in_tile[g] = x - own;
+        if (lane == 31) {
+            ranks.tile[blockIdx.x] = x;
+            __threadfence();
+            last = atomicAdd(&bst->done, 1) == (int)gridDim.x - 1;
+            if (last) bst->done = 0;  // for the next level
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // the tiles' exclusive scan, kPer consecutive tiles a thread
+    constexpr int kPer = 8;
+    int carry = 0;
+    for (int t0 = 0; t0 < (int)gridDim.x; t0 += kFlagThreads * kPer) {
+        const int b = t0 + threadIdx.x * kPer;
+        int v[kPer], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            v[j] = b + j < (int)gridDim.x ? __ldcg(&ranks.tile[b + j]) : 0;
+            sum += v[j];
+        }
+        int x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        __syncthreads();  // wc: its last readers are through
+        if (lane == 31) wc[warp] = x;
+        __syncthreads();
+        int run = carry + x - sum;
+        for (int w = 0; w < kWarps; ++w) {
+            if (w < warp) run += wc[w];
+            carry += wc[w];
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (b + j < (int)gridDim.x) ranks.tile[b + j] = run;
+            run += v[j];
+        }
+    }
+}
+
+// Children of every active segment: the two nodes (at depth level + 1), and for each child of more
+// than kFinishSlots triangles a slot of the next level (allocated with an atomic counter, its box
+// cleared); a child of K < size <= kFinishSlots triangles goes to the small list {start, end, node,
+// depth} that k_split_finish completes. part[s] = {start, middle, left rank of the start};
+// child_next[s] = the children's slots of the next level, -2 for a small child or -1 for a leaf.
+// The order of segments in either list is immaterial: positions come from the node ranges alone.
+__global__ void k_split_children(BuildState* __restrict__ bst, LevelBound lb, int K,
                                  const int* __restrict__ s_start, const int* __restrict__ s_end,
-                                 const int* __restrict__ s_node, const int* __restrict__ lf,
+                                 const int* __restrict__ s_node, LeftRanks ranks,
                                  int* __restrict__ nfirst, int* __restrict__ nlast,
                                  int* __restrict__ nparent, int* __restrict__ nleft,
                                  int* __restrict__ nright, int* __restrict__ depth_of,
-                                 int* __restrict__ counts, int* __restrict__ n_start,
-                                 int* __restrict__ n_end, int* __restrict__ n_node,
-                                 unsigned* __restrict__ n_box, int4* __restrict__ small,
-                                 int* __restrict__ child_next) {
+                                 int* __restrict__ n_start, int* __restrict__ n_end,
+                                 int* __restrict__ n_node, unsigned* __restrict__ n_box,
+                                 int4* __restrict__ small, int4* __restrict__ part,
+                                 int2* __restrict__ child_next) {
     const int sg = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nact = level_segments(bst, lb), node_base = bst->level[lb.level].y;
+    if (sg == 0) {
+        if (nact != bst->level[lb.level].x) atomicOr(&bst->status, ST_BUILD_BOUND);
+        bst->level[lb.level + 1].y = node_base + 2 * nact;
+        bst->internal[lb.level] = nact;
+    }
     if (sg >= nact) return;
-    const int b = s_start[sg], e = s_end[sg], mid = b + (lf[e] - lf[b]);
+    const int b = s_start[sg], e = s_end[sg], fb = left_rank(ranks, b);
+    const int mid = b + (left_rank(ranks, e) - fb);
     const int l = node_base + 2 * sg, r = l + 1, p = s_node[sg];
     nfirst[l] = b;
     nlast[l] = mid - 1;
@@ -863,61 +1020,57 @@ __global__ void k_split_children(int nact, int node_base, int level, int K,
     nleft[l] = nright[l] = nleft[r] = nright[r] = -1;
     nleft[p] = l;
     nright[p] = r;
-    depth_of[l] = depth_of[r] = level + 1;
+    depth_of[l] = depth_of[r] = lb.level + 1;
+    int next[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int cb = c == 0 ? b : mid, ce = c == 0 ? mid : e;
-        const int k = warp_append(&counts[0], ce - cb > kFinishSlots);
+        const int k = warp_append(&bst->level[lb.level + 1].x, ce - cb > kFinishSlots);
         if (k >= 0) {
             n_start[k] = cb;
             n_end[k] = ce;
             n_node[k] = l + c;
             box_clear_level(n_box, k);
         }
-        const int j = warp_append(&counts[1], ce - cb > K && ce - cb <= kFinishSlots);
-        if (j >= 0) small[j] = make_int4(cb, ce, l + c, level + 1);
-        child_next[2 * sg + c] = k >= 0 ? k : j >= 0 ? -2 : -1;
+        const int j = warp_append(&bst->small_len, ce - cb > K && ce - cb <= kFinishSlots);
+        if (j >= 0) small[j] = make_int4(cb, ce, l + c, lb.level + 1);
+        next[c] = k >= 0 ? k : j >= 0 ? -2 : -1;
     }
+    part[sg] = make_int4(b, mid, fb, 0);
+    child_next[sg] = make_int2(next[0], next[1]);
 }
 
 // Stable partition of every active segment: left-flagged slots first, each side in its order.
 // Slots of children that stay active go to the next level's buffers (and into their child's
 // box); those of leaves are final.
-__global__ void k_split_scatter(int64_t n, SplitSlots cur, SplitSlots nxt,
-                                const int* __restrict__ lf, const int* __restrict__ s_start,
-                                const int* __restrict__ s_end, const int* __restrict__ child_next,
-                                int* __restrict__ final_perm, unsigned* __restrict__ n_box,
-                                const int* __restrict__ next_count) {
+__global__ void k_split_scatter(int64_t n, const BuildState* __restrict__ bst, LevelBound lb,
+                                SplitSlots cur, SplitSlots nxt, LeftRanks ranks,
+                                const int4* __restrict__ part, const int2* __restrict__ child_next,
+                                int* __restrict__ final_perm, unsigned* __restrict__ n_box) {
+    if (level_segments(bst, lb) == 0) return;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int key = -1;
-    float cx = 0.f, cy = 0.f, cz = 0.f;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < n) {
         const int sg = cur.seg[i];
+        t = cur.tri[i];
+        const int rank = left_rank(ranks, (int)i);
+        const bool left = ranks.bits[i >> 5] >> (i & 31) & 1u;
         if (sg < 0) {
             nxt.seg[i] = -1;
         } else {
-            const int b = s_start[sg], e = s_end[sg];
-            const int fb = lf[b], nl = lf[e] - fb, left_before = lf[i] - fb;
-            const bool left = lf[i + 1] != lf[i];  // the exclusive scan steps where the flag is set
-            const int64_t dest = left ? b + left_before : b + nl + ((int)(i - b) - left_before);
-            const int k = child_next[2 * sg + (left ? 0 : 1)];
-            if (k >= 0 || k == -2) {  // active next level, or a small segment's slots
-                cx = cur.cx[i];
-                cy = cur.cy[i];
-                cz = cur.cz[i];
-                nxt.perm[dest] = cur.perm[i];
-                nxt.cx[dest] = cx;
-                nxt.cy[dest] = cy;
-                nxt.cz[dest] = cz;
-                nxt.seg[dest] = k >= 0 ? k : -1;
-                key = k >= 0 ? k : -1;
-            } else {
-                final_perm[dest] = cur.perm[i];
-                nxt.seg[dest] = -1;
-            }
+            const int4 sp = part[sg];
+            const int2 cn = child_next[sg];
+            const int left_before = rank - sp.z;
+            const int64_t dest = left ? sp.x + left_before : sp.y + ((int)(i - sp.x) - left_before);
+            const int k = left ? cn.x : cn.y;
+            if (k != -1) nxt.tri[dest] = t;  // active next level, or a small segment's slots
+            else final_perm[dest] = __float_as_int(t.w);
+            key = k >= 0 ? k : -1;
+            nxt.seg[dest] = key;
         }
     }
-    box_add(key, cx, cy, cz, n_box + box_copy_offset(*next_count <= kBoxCopyKeys));
+    box_add(key, t.x, t.y, t.z, n_box + box_copy_offset(bst->level[lb.level + 1].x <= kBoxCopyKeys));
 }
 
 // A small segment in shared memory. Sub-segments are named by their first position, so a
@@ -974,13 +1127,14 @@ __device__ void block_exclusive_scan(int* a, int count, int* wsum) {
 // by split by the level loop's rules (split_decide and the flags, children and stable partition
 // of k_split_flags / k_split_children / k_split_scatter) in shared memory. The slots are in A for
 // an even depth and in B for an odd one (the level that made the segment wrote them there, and
-// later levels write only other segments' ranges). Each step's node ids are one allocation from
-// node_count.
+// later levels write only other segments' ranges). Each step's node ids are one allocation after
+// the level loop's nodes.
 __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
-    const int4* __restrict__ small, SplitSlots A, SplitSlots B, int K, int* __restrict__ node_count,
-    int cap, int* __restrict__ nfirst, int* __restrict__ nlast, int* __restrict__ nparent,
-    int* __restrict__ nleft, int* __restrict__ nright, int* __restrict__ depth_of,
-    int* __restrict__ final_perm, unsigned* __restrict__ status) {
+    const int4* __restrict__ small, SplitSlots A, SplitSlots B, int K, BuildState* __restrict__ bst,
+    int level_nodes, int cap, int* __restrict__ nfirst, int* __restrict__ nlast,
+    int* __restrict__ nparent, int* __restrict__ nleft, int* __restrict__ nright,
+    int* __restrict__ depth_of, int* __restrict__ final_perm) {
+    unsigned* status = &bst->status;
     extern __shared__ __align__(16) unsigned char finish_smem[];
     FinishShared& S = *reinterpret_cast<FinishShared*>(finish_smem);
     const int4 seg = small[blockIdx.x];
@@ -991,10 +1145,11 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
     }
     const SplitSlots& X = (d0 & 1) ? B : A;
     for (int i = tid; i < size; i += kFinishThreads) {
-        S.c[0][i] = X.cx[gb + i];
-        S.c[1][i] = X.cy[gb + i];
-        S.c[2][i] = X.cz[gb + i];
-        S.perm[i] = X.perm[gb + i];
+        const float4 t = X.tri[gb + i];
+        S.c[0][i] = t.x;
+        S.c[1][i] = t.y;
+        S.c[2][i] = t.z;
+        S.perm[i] = __float_as_int(t.w);
         S.orig[0][i] = (unsigned short)i;
         S.sid[0][i] = 0;
     }
@@ -1041,7 +1196,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
         // after the flags, so the block does not wait for it at the next barrier
         int nb = 0;
         if (tid == 0) {
-            nb = atomicAdd(node_count, 2 * ns);
+            nb = level_nodes + atomicAdd(&bst->finish_nodes, 2 * ns);
+            atomicAdd(&bst->internal[depth], ns);
             S.rank = 0;
             S.ns[cur ^ 1] = 0;
         }
@@ -1622,8 +1778,6 @@ constexpr int kLaneLevel = 8192;
 // child), by an integer ascent from the emitted leaves (the second child to arrive continues);
 // the FP64 combine then runs height by height over dense lists (k_refit_level), like the split
 // tree's levels, instead of on the ascent's ever sparser warps.
-constexpr int kMaxHeight = 4 * 64 + 64;  // key bits + index bits bound the depth
-
 __global__ void k_heights(int num_leaves, const int* __restrict__ leaf_list,
                           const uint64_t* __restrict__ keys, const int* __restrict__ parent,
                           const int* __restrict__ first, const int* __restrict__ last,
@@ -1677,16 +1831,6 @@ __global__ void k_height_hist(int nint, const uint64_t* __restrict__ keys,
     __syncthreads();
     for (int i = threadIdx.x; i < kMaxHeight; i += blockDim.x)
         if (h_s[i]) atomicAdd(&hist[i], h_s[i]);
-}
-
-__global__ void k_height_offsets(int* __restrict__ hist) {  // one thread: exclusive scan in place
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int acc = 0;
-    for (int i = 0; i < kMaxHeight; ++i) {
-        const int c = hist[i];
-        hist[i] = acc;
-        acc += c;
-    }
 }
 
 __global__ void k_height_sort(int nint, const uint64_t* __restrict__ keys,
@@ -2075,6 +2219,47 @@ __global__ void k_tri_records(int n, const uint32_t* __restrict__ tri_of_slot,
     sorted_tri[s] = (int)t;
 }
 
+// Reads the build's device state back: request copies it (in stream order) into one of two pinned
+// slots of the calling thread, wait returns that slot once the copy is in. The destructor waits
+// for what is outstanding, so that a build that stops early leaves no copy behind.
+class StateReader {
+public:
+    StateReader(const BuildState* src, cudaStream_t s) : src_(src), s_(s) {
+        struct Slots {
+            BuildState* p = nullptr;
+            ~Slots() {
+                if (p) cudaFreeHost(p);
+            }
+        };
+        thread_local Slots t;
+        if (!t.p) FWN_CUDA_CHECK(cudaHostAlloc(&t.p, 2 * sizeof(BuildState), cudaHostAllocPortable));
+        slots_ = t.p;
+        for (cudaEvent_t& e : ev_) FWN_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    StateReader(const StateReader&) = delete;
+    ~StateReader() {
+        for (cudaEvent_t e : ev_)
+            if (e) {
+                cudaEventSynchronize(e);
+                cudaEventDestroy(e);
+            }
+    }
+    void request(int k) {
+        FWN_CUDA_CHECK(cudaMemcpyAsync(&slots_[k], src_, sizeof(BuildState), cudaMemcpyDeviceToHost, s_));
+        FWN_CUDA_CHECK(cudaEventRecord(ev_[k], s_));
+    }
+    const BuildState& wait(int k) {
+        FWN_CUDA_CHECK(cudaEventSynchronize(ev_[k]));
+        return slots_[k];
+    }
+
+private:
+    const BuildState* src_;
+    cudaStream_t s_;
+    BuildState* slots_ = nullptr;
+    cudaEvent_t ev_[2] = {};
+};
+
 // Build temporaries come from the library's build pool, which keeps freed memory mapped across
 // synchronisations (up to kBuildRetainBytes): a rebuild, or the next mesh of a batch, reuses it
 // instead of mapping gigabytes of new pages (the device's default pool returns freed memory at
@@ -2120,8 +2305,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     FWN_CUDA_CHECK(cudaMalloc(&e.meshes, nmeshes * sizeof(MeshInfo)));
     e.meshes_h = new MeshInfo[nmeshes];
     unsigned* enc = dalloc<unsigned>(6 * nmeshes, st);
-    unsigned* status = dalloc<unsigned>(1, st);
-    FWN_CUDA_CHECK(cudaMemsetAsync(status, 0, sizeof(unsigned), st));
+    BuildState* bst = dalloc<BuildState>(1, st);
+    unsigned* status = &bst->status;
+    FWN_CUDA_CHECK(cudaMemsetAsync(bst, 0, sizeof(BuildState), st));
     k_init_bbox<<<grid_for(6 * nmeshes, 256), 256, 0, st>>>(enc, (int)nmeshes);
     int64_t maxv = 0;
     for (int64_t m = 0; m < nmeshes; ++m) maxv = std::max(maxv, voff_h[m + 1] - voff_h[m]);
@@ -2146,7 +2332,7 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     track(voff);
     track(foff);
     track(enc);
-    track(status);
+    track(bst);
 
     if (nf > 0) {
         const int n = (int)nf;
@@ -2174,11 +2360,10 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         const uint32_t* tri_of_slot = nullptr;
         int num_nodes = 0;
         unsigned st_h = 0;
+        std::vector<int> h_hist(kMaxHeight);  // internal nodes by depth or height
         // split tree: every node's depth (roots 0), the order of the level-by-level refit
         int* depth_of = split ? (int*)track(dalloc<int>(cap, st)) : nullptr;
-        auto check_input = [&]() {
-            FWN_CUDA_CHECK(cudaMemcpyAsync(&st_h, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+        auto check_input = [](unsigned st_h) {
             if (st_h & ST_BAD_INDEX) throw Error(FWN_INVALID_ARG, "triangle vertex index out of range");
             if (st_h & ST_NONFINITE)
                 throw Error(FWN_INVALID_ARG, "non-finite vertex coordinate referenced by a triangle");
@@ -2196,7 +2381,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             k_tri_keys<<<grid_for(n, 256), 256, 0, st>>>(d_V, d_F, voff, foff, (int)nmeshes, nf,
                                                          e.meshes, keys_a, vals_a, status);
             FWN_CUDA_CHECK(cudaGetLastError());
-            check_input();
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&st_h, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+            check_input(st_h);
             const bool in_b = radix_sort_u64(keys_a, vals_a, keys_b, vals_b, n,
                                              MORTON_BITS + mesh_bits, sort_tmp, st);
             keys = in_b ? keys_b : keys_a;
@@ -2251,15 +2438,16 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             int* final_perm = (int*)track(dalloc<int>(n, st));
             SplitSlots A, B;
             for (SplitSlots* X : {&A, &B}) {
-                X->perm = (int*)track(dalloc<int>(n, st));
-                X->cx = (float*)track(dalloc<float>(n, st));
-                X->cy = (float*)track(dalloc<float>(n, st));
-                X->cz = (float*)track(dalloc<float>(n, st));
+                X->tri = (float4*)track(dalloc<float4>(n, st));
                 X->seg = (int*)track(dalloc<int>(n, st));
             }
-            int* lflags = (int*)track(dalloc<int>(n + 1, st));
-            int* child_next = (int*)track(dalloc<int>(2 * (size_t)smax, st));
-            int* counts = (int*)track(dalloc<int>(3, st));  // next level, small list, node ids
+            const int tiles = n / kSplitTile + 1;  // slots 0 .. n: entry n ends the last rank
+            LeftRanks ranks;
+            ranks.bits = (unsigned*)track(dalloc<unsigned>(n / 32 + 1, st));
+            ranks.in_tile = (int*)track(dalloc<int>(n / 32 + 1, st));
+            ranks.tile = (int*)track(dalloc<int>(tiles, st));
+            int4* part = (int4*)track(dalloc<int4>(smax, st));
+            int2* child_next = (int2*)track(dalloc<int2>(smax, st));
             int4* small = (int4*)track(dalloc<int4>(smax, st));
             if (!h_small.empty())
                 FWN_CUDA_CHECK(cudaMemcpyAsync(small, h_small.data(), h_small.size() * sizeof(int4),
@@ -2308,75 +2496,84 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                                            d_mesh_seg, A, final_perm, skeys, box_a,
                                                            nact <= kBoxCopyKeys, status);
             FWN_CUDA_CHECK(cudaGetLastError());
-            check_input();
-            int node_base = nroots;
+            // A mesh of m triangles has segments to split for at least log2(m / kFinishSlots)
+            // levels: the host launches those without looking. From there on level l + 1 is
+            // launched before level l's counts have come back: the kernels of a level without
+            // segments return at once, and the host's round trip (18 us a level, measured) runs
+            // beside the next level.
+            int sure = 0;  // levels that have segments whatever the splits
+            for (size_t k = 0; k < s_start.size(); ++k)
+                while ((int64_t)kFinishSlots << sure < s_end[k] - s_start[k]) ++sure;
+            const int2 level0 = make_int2(nact, nroots);
             int nsmall = (int)h_small.size();
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&bst->level[0], &level0, sizeof(level0),
+                                           cudaMemcpyHostToDevice, st));
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&bst->small_len, &nsmall, sizeof(int),
+                                           cudaMemcpyHostToDevice, st));
             SplitSlots* cur = &A;
             SplitSlots* nxt = &B;
-            int level = 0;
-            while (nact > 0) {
-                if (level > kSpatialLevels + 64)  // position splits halve every segment
-                    throw Error(FWN_INTERNAL, "split build did not converge");
-                if (node_base + 2 * nact > cap) throw Error(FWN_INTERNAL, "split build node overflow");
-                if (nact > seg_bound) throw Error(FWN_INTERNAL, "split build segment overflow");
-                k_split_decide<<<grid_for(nact, 128), 128, 0, st>>>(
-                    nact, level >= kSpatialLevels, box_a, axis_of, split_of, spatial_of, seg_box);
-                if (binned && level < kSpatialLevels) {  // the binned plane of each segment
-                    const int words = nact * kSegBinWords;
-                    k_split_bins_init<<<grid_for(words, 256), 256, 0, st>>>(words, bins);
-                    k_split_bins<<<(int)((n + kBinChunk - 1) / kBinChunk), 256, 0, st>>>(
-                        n, *cur, seg_box, bins, status);
-                    k_split_choose<<<grid_for(32 * nact, 128), 128, 0, st>>>(nact, seg_box, bins,
-                                                                             axis_of, bin_of,
-                                                                             spatial_of);
+            StateReader reader(bst, st);
+            if (nact == 0) {
+                reader.request(0);
+                check_input(reader.wait(0).status);
+            }
+            int levels = 0;  // levels with segments
+            for (int level = 0; nact > 0; ++level) {
+                const LevelBound lb{level, cap, seg_bound};
+                const int most = (int)std::min<int64_t>(seg_bound, (int64_t)nact << std::min(level, 30));
+                if (binned) {
+                    k_split_decide<<<grid_for(most, 128), 128, 0, st>>>(
+                        bst, lb, box_a, axis_of, split_of, spatial_of, seg_box);
+                    if (level < kSpatialLevels) {  // the binned plane of each segment
+                        k_split_bins_init<<<grid_for((int64_t)most * kSegBinWords, 256), 256, 0, st>>>(
+                            bst, lb, bins);
+                        k_split_bins<<<(int)((n + kBinChunk - 1) / kBinChunk), 256, 0, st>>>(
+                            n, bst, lb, *cur, seg_box, bins);
+                        k_split_choose<<<grid_for(32 * (int64_t)most, 128), 128, 0, st>>>(
+                            bst, lb, seg_box, bins, axis_of, bin_of, spatial_of);
+                    }
                 }
-                k_split_flags<<<grid_for(n + 1, 256), 256, 0, st>>>(n, *cur, seg_a[0], seg_a[1],
-                                                                   axis_of, split_of, spatial_of,
-                                                                   bin_of, seg_box, lflags);
-                exclusive_scan_i32(lflags, n + 1, scan_tmp, st);
-                const int h_counts[2] = {0, nsmall};
-                FWN_CUDA_CHECK(cudaMemcpyAsync(counts, h_counts, sizeof(h_counts),
-                                               cudaMemcpyHostToDevice, st));
-                k_split_children<<<grid_for(nact, 128), 128, 0, st>>>(
-                    nact, node_base, level, K, seg_a[0], seg_a[1], seg_a[2], lflags, first, last,
-                    parent, left, right, depth_of, counts, seg_b[0], seg_b[1], seg_b[2], box_b,
-                    small, child_next);
-                // lflags now holds the exclusive scan of the left flags (a slot's flag is the
-                // step from its entry to the next)
-                k_split_scatter<<<grid_for(n, 256), 256, 0, st>>>(n, *cur, *nxt, lflags, seg_a[0],
-                                                                 seg_a[1], child_next, final_perm,
-                                                                 box_b, counts);
+                (binned ? k_split_flags<true> : k_split_flags<false>)<<<tiles, kFlagThreads, 0, st>>>(
+                    n, bst, lb, *cur, seg_a[0], seg_a[1], box_a, axis_of, split_of, spatial_of,
+                    bin_of, seg_box, ranks);
+                k_split_children<<<grid_for(most, 128), 128, 0, st>>>(
+                    bst, lb, K, seg_a[0], seg_a[1], seg_a[2], ranks, first, last, parent, left,
+                    right, depth_of, seg_b[0], seg_b[1], seg_b[2], box_b, small, part, child_next);
+                k_split_scatter<<<grid_for(n, 256), 256, 0, st>>>(n, bst, lb, *cur, *nxt, ranks, part,
+                                                                 child_next, final_perm, box_b);
                 FWN_CUDA_CHECK(cudaGetLastError());
-                node_base += 2 * nact;
-                int next[2] = {0, 0};
-                FWN_CUDA_CHECK(cudaMemcpyAsync(next, counts, sizeof(next), cudaMemcpyDeviceToHost,
-                                               st));
-                FWN_CUDA_CHECK(cudaStreamSynchronize(st));
-                nact = next[0];
-                nsmall = next[1];
-                ++level;
+                if (level + 1 >= sure) reader.request(level & 1);
+                if (level >= sure) {
+                    const BuildState& h = reader.wait((level - 1) & 1);
+                    check_input(h.status);
+                    if (h.status & ST_BUILD_BOUND)
+                        throw Error(FWN_INTERNAL, "split build passed its node or depth bound");
+                    nsmall = h.small_len;
+                    levels = level;
+                    if (h.level[level].x == 0) break;
+                    if (level > kSpatialLevels + 64)  // position splits halve every segment
+                        throw Error(FWN_INTERNAL, "split build did not converge");
+                }
                 std::swap(cur, nxt);
                 std::swap(box_a, box_b);
                 for (int k = 0; k < 3; ++k) std::swap(seg_a[k], seg_b[k]);
             }
+            const int level_nodes = nact ? reader.wait((levels - 1) & 1).level[levels].y : nroots;
             if (nsmall > 0) {  // the small segments' subtrees, one block each
-                FWN_CUDA_CHECK(cudaMemcpyAsync(counts + 2, &node_base, sizeof(int),
-                                               cudaMemcpyHostToDevice, st));
                 FWN_CUDA_CHECK(cudaFuncSetAttribute(k_split_finish,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)sizeof(FinishShared)));
                 k_split_finish<<<nsmall, kFinishThreads, sizeof(FinishShared), st>>>(
-                    small, A, B, K, counts + 2, cap, first, last, parent, left, right, depth_of,
-                    final_perm, status);
+                    small, A, B, K, bst, level_nodes, cap, first, last, parent, left, right, depth_of,
+                    final_perm);
                 FWN_CUDA_CHECK(cudaGetLastError());
-                FWN_CUDA_CHECK(cudaMemcpyAsync(&node_base, counts + 2, sizeof(int),
-                                               cudaMemcpyDeviceToHost, st));
-                FWN_CUDA_CHECK(cudaMemcpyAsync(&st_h, status, sizeof(unsigned),
-                                               cudaMemcpyDeviceToHost, st));
-                FWN_CUDA_CHECK(cudaStreamSynchronize(st));
-                if ((st_h & ST_BUILD_BOUND) || node_base > cap)
-                    throw Error(FWN_INTERNAL, "split build passed its node or depth bound");
             }
+            reader.request(0);
+            const BuildState& h = reader.wait(0);
+            const int node_base = level_nodes + h.finish_nodes;
+            if ((h.status & ST_BUILD_BOUND) || node_base > cap)
+                throw Error(FWN_INTERNAL, "split build passed its node or depth bound");
+            std::copy(h.internal, h.internal + kMaxHeight, h_hist.begin());
             num_nodes = node_base;
             keys = skeys;
             tri_of_slot = reinterpret_cast<const uint32_t*>(final_perm);
@@ -2391,10 +2588,14 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                                                        pos, skip, e.meshes);
             FWN_CUDA_CHECK(cudaGetLastError());
         }
-        int E = 0, NL = 0;
-        FWN_CUDA_CHECK(cudaMemcpyAsync(&E, cnt + n, sizeof(int), cudaMemcpyDeviceToHost, st));
-        FWN_CUDA_CHECK(cudaMemcpyAsync(&NL, leaf_list_len, sizeof(int), cudaMemcpyDeviceToHost, st));
-        FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+        int E = num_nodes, NL = 0;
+        if (split) {  // every node is emitted, and all but the internal ones are leaves
+            NL = num_nodes - std::accumulate(h_hist.begin(), h_hist.end(), 0);
+        } else {
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&E, cnt + n, sizeof(int), cudaMemcpyDeviceToHost, st));
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&NL, leaf_list_len, sizeof(int), cudaMemcpyDeviceToHost, st));
+            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+        }
         e.num_nodes = E;
 
         NvtxRange trace_refit("fwn build: FP64 refit, radii, records");
@@ -2433,20 +2634,21 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                 k_heights<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_list, keys, parent, first,
                                                              last, visit, key, status);
             }
-            int* hist = (int*)track(dalloc<int>(kMaxHeight, st));
+            int* offsets = (int*)track(dalloc<int>(kMaxHeight, st));
             int* order = (int*)track(dalloc<int>(count, st));
-            FWN_CUDA_CHECK(cudaMemsetAsync(hist, 0, kMaxHeight * sizeof(int), st));
-            k_height_hist<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
-                                                                hist, status);
-            std::vector<int> h_hist(kMaxHeight);
-            FWN_CUDA_CHECK(cudaMemcpyAsync(h_hist.data(), hist, kMaxHeight * sizeof(int),
-                                           cudaMemcpyDeviceToHost, st));
-            k_height_offsets<<<1, 32, 0, st>>>(hist);
-            k_height_sort<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
-                                                                hist, order);
-            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+            if (!split) {
+                k_height_hist<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
+                                                                    bst->internal, status);
+                FWN_CUDA_CHECK(cudaMemcpyAsync(h_hist.data(), bst->internal, kMaxHeight * sizeof(int),
+                                               cudaMemcpyDeviceToHost, st));
+                FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+            }
             std::vector<int> off(kMaxHeight + 1, 0);
             for (int h = 0; h < kMaxHeight; ++h) off[h + 1] = off[h] + h_hist[h];
+            FWN_CUDA_CHECK(cudaMemcpyAsync(offsets, off.data(), kMaxHeight * sizeof(int),
+                                           cudaMemcpyHostToDevice, st));
+            k_height_sort<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
+                                                                offsets, order);
             for (int t = 0; t < kMaxHeight; ++t) {
                 const int h = split ? kMaxHeight - 1 - t : t;
                 if (h_hist[h] == 0) continue;
