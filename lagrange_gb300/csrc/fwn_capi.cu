@@ -20,11 +20,12 @@ void set_last_error(const std::string& m) { g_last_error = m; }
 namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mutex;
-// two pools per device, created on first use and kept for the process lifetime: one for query
-// scratch, one for build temporaries, so that the gigabytes a large build frees (in block sizes
-// of its own) never stand in for a query's scratch and push the query pool over its threshold
-cudaMemPool_t g_pools[2][kMaxDevices] = {};
-constexpr uint64_t kRetain[2] = {kScratchRetainBytes, kBuildRetainBytes};
+// three pools per device, created on first use and kept for the process lifetime: one for query
+// scratch, one for build temporaries, one for the engines' own memory, so that the gigabytes a
+// large build frees (in block sizes of its own) never stand in for a query's scratch and push the
+// query pool over its threshold
+cudaMemPool_t g_pools[3][kMaxDevices] = {};
+constexpr uint64_t kRetain[3] = {kScratchRetainBytes, kBuildRetainBytes, kEngineRetainBytes};
 
 cudaMemPool_t scratch_pool(int dev, int kind) {
     if (dev < 0 || dev >= kMaxDevices) throw Error(FWN_INTERNAL, "device ordinal out of range");
@@ -91,18 +92,25 @@ void* scratch_alloc(size_t bytes, cudaStream_t st) { return pool_alloc(bytes, st
 
 void* build_alloc(size_t bytes, cudaStream_t st) { return pool_alloc(bytes, st, 1); }
 
+void* engine_alloc(size_t bytes, cudaStream_t st) {
+    return bytes ? pool_alloc(bytes, st, 2) : nullptr;
+}
+
 Engine::~Engine() {
     // free on the engine's device, then give the caller back its current device
     int cur = -1;
     const bool swap = cudaGetDevice(&cur) == cudaSuccess && cur != device &&
                       cudaSetDevice(device) == cudaSuccess;
-    if (nodes32) cudaFree(nodes32);
-    if (nodes64) cudaFree(nodes64);
-    if (soa) cudaFree(soa);
-    if (tris) cudaFree(tris);
-    if (sorted_tri) cudaFree(sorted_tri);
-    if (meshes) cudaFree(meshes);
-    if (stage) cudaFree(stage);
+    // work that still reads the engine may be in flight on any stream: wait for the device, as
+    // cudaFree does (which takes over where the device cannot be waited for)
+    void* own[] = {nodes32, nodes64, soa, tris, sorted_tri, meshes, stage};
+    bool waited = false, idle = false;
+    for (void* p : own) {
+        if (!p) continue;
+        if (!waited) idle = cudaDeviceSynchronize() == cudaSuccess;
+        waited = true;
+        if (!(idle && cudaFreeAsync(p, cudaStreamPerThread) == cudaSuccess)) cudaFree(p);
+    }
     if (swap) cudaSetDevice(cur);
     delete[] meshes_h;
     delete[] node_tri_begin_h;

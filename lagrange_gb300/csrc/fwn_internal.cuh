@@ -160,6 +160,11 @@ void* scratch_alloc(size_t bytes, cudaStream_t stream);
 // kBuildRetainBytes mapped for the next build (a 42M-triangle forest's are ~10 GB).
 constexpr uint64_t kBuildRetainBytes = uint64_t(12) << 30;
 void* build_alloc(size_t bytes, cudaStream_t stream);
+// Engines live in a third pool: mapping and unmapping a 2-million-triangle engine's 190 MB with
+// cudaMalloc and cudaFree took 0.5 ms of a 3.8 ms build, query and destroy. A destroyed engine's
+// memory goes to the next one; the pool keeps at most kEngineRetainBytes that no engine uses.
+constexpr uint64_t kEngineRetainBytes = uint64_t(2) << 30;
+void* engine_alloc(size_t bytes, cudaStream_t stream);
 
 struct Scratch {
     void* p = nullptr;

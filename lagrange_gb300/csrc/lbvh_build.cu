@@ -283,12 +283,26 @@ __device__ __forceinline__ int block_append(int* __restrict__ counter, bool pred
     return at;
 }
 
+// Leaves listed for the refit, counted by size (every thread of the block calls it).
+constexpr int kLeafSizes = 17;  // triangles of a leaf: 0 .. WARP_LEAF_MAX (0 does not occur)
+__device__ __forceinline__ int leaf_size_of(int first, int last) {
+    return min(max(last - first + 1, 0), kLeafSizes - 1);
+}
+__device__ __forceinline__ void block_count_leaf(bool leaf, int size, int* __restrict__ by_size) {
+    __shared__ int h[kLeafSizes];
+    if (threadIdx.x < kLeafSizes) h[threadIdx.x] = 0;
+    __syncthreads();
+    if (leaf) atomicAdd(&h[size], 1);
+    __syncthreads();
+    if (threadIdx.x < kLeafSizes && h[threadIdx.x]) atomicAdd(&by_size[threadIdx.x], h[threadIdx.x]);
+}
+
 // flags: bit0 emitted, bit1 leaf
 __global__ void k_emit_count(int n, int K, const uint64_t* __restrict__ keys,
                              const int* __restrict__ parent, const int* __restrict__ first,
                              const int* __restrict__ last, int* __restrict__ cnt_first,
                              uint8_t* __restrict__ flags, int* __restrict__ leaf_list,
-                             int* __restrict__ leaf_list_len) {
+                             int* __restrict__ leaf_list_len, int* __restrict__ by_size) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     bool pred = false;
     if (u < 2 * n - 1) {
@@ -303,6 +317,7 @@ __global__ void k_emit_count(int n, int K, const uint64_t* __restrict__ keys,
     // thread each; the list order does not matter (each node's arithmetic is fixed)
     const int at = block_append(leaf_list_len, pred);
     if (at >= 0) leaf_list[at] = u;
+    block_count_leaf(pred, pred ? leaf_size_of(first[u], last[u]) : 0, by_size);
 }
 
 __global__ void k_positions(int num_nodes, const int* __restrict__ parent,
@@ -397,6 +412,12 @@ struct BuildState {
     int small_len;             // small segments listed
     int finish_nodes;          // nodes made by k_split_finish
     int done;                  // blocks of the running k_split_flags that are through
+    int emitted;               // nodes of the final tree (LBVH)
+    int leaf_list;             // leaves listed for the refit
+    int leaf_count;            // leaves among the records
+    int radius_list;           // nodes listed for k_node_radius_small
+    int leaf_size[kLeafSizes]; // listed leaves by triangle count
+    int leaf_next[kLeafSizes]; // of those, the ones k_leaf_sort has placed
     int2 level[kMaxLevels + 1];  // active segments; nodes made before
     int internal[kMaxHeight];  // internal nodes by depth (split) or height (LBVH)
 };
@@ -1284,9 +1305,10 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
 // Node flags of the split tree (every node emitted; leaves = no children), the per-first-slot
 // node counts of the position scan, and the refit's leaf list.
 __global__ void k_split_emit(int num_nodes, const int* __restrict__ nfirst,
-                             const int* __restrict__ nleft, uint8_t* __restrict__ flags,
-                             int* __restrict__ cnt_first, int* __restrict__ leaf_list,
-                             int* __restrict__ leaf_list_len) {
+                             const int* __restrict__ nlast, const int* __restrict__ nleft,
+                             uint8_t* __restrict__ flags, int* __restrict__ cnt_first,
+                             int* __restrict__ leaf_list, int* __restrict__ leaf_list_len,
+                             int* __restrict__ by_size) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     bool leaf = false;
     if (u < num_nodes) {
@@ -1296,6 +1318,7 @@ __global__ void k_split_emit(int num_nodes, const int* __restrict__ nfirst,
     }
     const int at = block_append(leaf_list_len, leaf);
     if (at >= 0) leaf_list[at] = u;
+    block_count_leaf(leaf, leaf ? leaf_size_of(nfirst[u], nlast[u]) : 0, by_size);
 }
 
 __global__ void k_split_mesh_roots(int nmeshes, const int* __restrict__ root_node,
@@ -1615,39 +1638,11 @@ __global__ void k_refit(int num_leaves, const int* __restrict__ leaf_list,
     store_rec(&stage[pos[e]], R);
 }
 
-// The refit's leaf list grouped by triangle count (a counting sort over 1..16), so that the 32
-// leaves of a warp run the same number of triangle iterations: the FP64 pipe costs the same for
-// a warp instruction whatever the number of active lanes.
-constexpr int kLeafSizes = 17;  // counts 0..16 (WARP_LEAF_MAX); 0 does not occur
-
-__device__ __forceinline__ int leaf_size_of(const int* __restrict__ first,
-                                            const int* __restrict__ last, int u) {
-    return min(max(last[u] - first[u] + 1, 0), kLeafSizes - 1);
-}
-
-__global__ void k_leaf_hist(int nl, const int* __restrict__ leaves, const int* __restrict__ first,
-                            const int* __restrict__ last, int* __restrict__ hist) {
-    __shared__ int h[kLeafSizes];
-    if (threadIdx.x < kLeafSizes) h[threadIdx.x] = 0;
-    __syncthreads();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nl) atomicAdd(&h[leaf_size_of(first, last, leaves[k])], 1);
-    __syncthreads();
-    if (threadIdx.x < kLeafSizes && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
-}
-
-__global__ void k_leaf_offsets(int* __restrict__ hist) {  // one thread: exclusive scan in place
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int acc = 0;
-    for (int i = 0; i < kLeafSizes; ++i) {
-        const int c = hist[i];
-        hist[i] = acc;
-        acc += c;
-    }
-}
-
+// The refit's leaf list grouped by triangle count (a counting sort over the sizes that the list's
+// maker counted), so that the 32 leaves of a warp run the same number of triangle iterations: the
+// FP64 pipe costs the same for a warp instruction whatever the number of active lanes.
 __global__ void k_leaf_sort(int nl, const int* __restrict__ leaves, const int* __restrict__ first,
-                            const int* __restrict__ last, int* __restrict__ offset,
+                            const int* __restrict__ last, BuildState* __restrict__ bst,
                             int* __restrict__ sorted) {
     __shared__ int cnt[kLeafSizes];   // the block's leaves per size (ranks from shared atomics)
     __shared__ int base[kLeafSizes];  // where they go: one global atomic per non-zero size
@@ -1657,12 +1652,15 @@ __global__ void k_leaf_sort(int nl, const int* __restrict__ leaves, const int* _
     int u = -1, sz = 0, rank = 0;
     if (k < nl) {
         u = leaves[k];
-        sz = leaf_size_of(first, last, u);
+        sz = leaf_size_of(first[u], last[u]);
         rank = atomicAdd(&cnt[sz], 1);
     }
     __syncthreads();
-    if (threadIdx.x < kLeafSizes && cnt[threadIdx.x])
-        base[threadIdx.x] = atomicAdd(&offset[threadIdx.x], cnt[threadIdx.x]);
+    if (threadIdx.x < kLeafSizes && cnt[threadIdx.x]) {
+        int before = 0;
+        for (int i = 0; i < (int)threadIdx.x; ++i) before += bst->leaf_size[i];
+        base[threadIdx.x] = before + atomicAdd(&bst->leaf_next[threadIdx.x], cnt[threadIdx.x]);
+    }
     __syncthreads();
     if (u >= 0) sorted[base[sz] + rank] = u;
 }
@@ -1778,13 +1776,13 @@ constexpr int kLaneLevel = 8192;
 // child), by an integer ascent from the emitted leaves (the second child to arrive continues);
 // the FP64 combine then runs height by height over dense lists (k_refit_level), like the split
 // tree's levels, instead of on the ascent's ever sparser warps.
-__global__ void k_heights(int num_leaves, const int* __restrict__ leaf_list,
+__global__ void k_heights(const int* __restrict__ num_leaves, const int* __restrict__ leaf_list,
                           const uint64_t* __restrict__ keys, const int* __restrict__ parent,
                           const int* __restrict__ first, const int* __restrict__ last,
                           int* __restrict__ visit, int* __restrict__ height,
                           unsigned* __restrict__ status) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= num_leaves) return;
+    if (k >= *num_leaves) return;
     int v = leaf_list[k], h = 0;
     for (int guard = 0; v != 0; ++guard) {
         const int p = parent[v];
@@ -2220,19 +2218,25 @@ __global__ void k_tri_records(int n, const uint32_t* __restrict__ tri_of_slot,
 }
 
 // Reads the build's device state back: request copies it (in stream order) into one of two pinned
-// slots of the calling thread, wait returns that slot once the copy is in. The destructor waits
-// for what is outstanding, so that a build that stops early leaves no copy behind.
+// slots of the calling thread, wait returns that slot once the copy is in (8 us, against 16 us and
+// more for a copy to pageable memory, and everything in one). The destructor waits for what is
+// outstanding, so that a build that stops early leaves no copy behind.
 class StateReader {
 public:
+    static constexpr int64_t kMeshes = 64;  // MeshInfos a slot has room for
+    struct Slot {
+        BuildState state;
+        MeshInfo meshes[kMeshes];
+    };
     StateReader(const BuildState* src, cudaStream_t s) : src_(src), s_(s) {
         struct Slots {
-            BuildState* p = nullptr;
+            Slot* p = nullptr;
             ~Slots() {
                 if (p) cudaFreeHost(p);
             }
         };
         thread_local Slots t;
-        if (!t.p) FWN_CUDA_CHECK(cudaHostAlloc(&t.p, 2 * sizeof(BuildState), cudaHostAllocPortable));
+        if (!t.p) FWN_CUDA_CHECK(cudaHostAlloc(&t.p, 2 * sizeof(Slot), cudaHostAllocPortable));
         slots_ = t.p;
         for (cudaEvent_t& e : ev_) FWN_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
@@ -2244,29 +2248,66 @@ public:
                 cudaEventDestroy(e);
             }
     }
-    void request(int k) {
-        FWN_CUDA_CHECK(cudaMemcpyAsync(&slots_[k], src_, sizeof(BuildState), cudaMemcpyDeviceToHost, s_));
+    void request(int k, const MeshInfo* meshes = nullptr, int64_t count = 0) {
+        FWN_CUDA_CHECK(cudaMemcpyAsync(&slots_[k].state, src_, sizeof(BuildState), cudaMemcpyDeviceToHost, s_));
+        if (count)
+            FWN_CUDA_CHECK(cudaMemcpyAsync(slots_[k].meshes, meshes, count * sizeof(MeshInfo),
+                                           cudaMemcpyDeviceToHost, s_));
         FWN_CUDA_CHECK(cudaEventRecord(ev_[k], s_));
     }
     const BuildState& wait(int k) {
         FWN_CUDA_CHECK(cudaEventSynchronize(ev_[k]));
-        return slots_[k];
+        return slots_[k].state;
     }
+    const MeshInfo* meshes(int k) const { return slots_[k].meshes; }
 
 private:
     const BuildState* src_;
     cudaStream_t s_;
-    BuildState* slots_ = nullptr;
+    Slot* slots_ = nullptr;
     cudaEvent_t ev_[2] = {};
 };
 
 // Build temporaries come from the library's build pool, which keeps freed memory mapped across
 // synchronisations (up to kBuildRetainBytes): a rebuild, or the next mesh of a batch, reuses it
 // instead of mapping gigabytes of new pages (the device's default pool returns freed memory at
-// every synchronisation).
-template <class T> T* dalloc(size_t count, cudaStream_t s) {
-    return count ? static_cast<T*>(build_alloc(count * sizeof(T), s)) : nullptr;
-}
+// every synchronisation). Small ones share a block: the fifty calls to the pool of a small build
+// took longer than its kernels' launches. Freed in stream order when the build ends, however it
+// ends.
+class BuildArena {
+public:
+    explicit BuildArena(cudaStream_t s) : s_(s) {}
+    BuildArena(const BuildArena&) = delete;
+    ~BuildArena() {
+        for (void* p : blocks_) cudaFreeAsync(p, s_);
+    }
+    template <class T> T* take(size_t count) {  // 256 B aligned
+        const size_t bytes = (count * sizeof(T) + 255) / 256 * 256;
+        if (!bytes) return nullptr;
+        if (bytes > kBlock / 2) return static_cast<T*>(block(bytes));
+        if (bytes > left_) {
+            next_ = static_cast<char*>(block(kBlock));
+            left_ = kBlock;
+        }
+        T* p = reinterpret_cast<T*>(next_);
+        next_ += bytes;
+        left_ -= bytes;
+        return p;
+    }
+
+private:
+    static constexpr size_t kBlock = size_t(32) << 20;
+    void* block(size_t bytes) {
+        blocks_.reserve(blocks_.size() + 1);
+        void* p = build_alloc(bytes, s_);
+        blocks_.push_back(p);
+        return p;
+    }
+    cudaStream_t s_;
+    std::vector<void*> blocks_;
+    char* next_ = nullptr;
+    size_t left_ = 0;
+};
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
@@ -2284,6 +2325,10 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     const int64_t nv = voff_h[nmeshes], nf = foff_h[nmeshes];
     if (nf > (int64_t)0x3fffffff)
         throw Error(FWN_INVALID_ARG, "at most 2^30-1 triangles per forest");
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    FWN_CUDA_CHECK(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone)
+        throw Error(FWN_CUDA_ERROR, "a build waits for its stream, which is being captured");
     e.nv = nv;
     e.nf = nf;
     e.nmeshes = nmeshes;
@@ -2296,16 +2341,18 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     FWN_CUDA_CHECK(cudaEventCreate(&ev1));
     FWN_CUDA_CHECK(cudaEventRecord(ev0, st));
 
-    int64_t* voff = dalloc<int64_t>(nmeshes + 1, st);
-    int64_t* foff = dalloc<int64_t>(nmeshes + 1, st);
+    BuildArena arena(st);
+    int64_t* voff = arena.take<int64_t>(nmeshes + 1);
+    int64_t* foff = arena.take<int64_t>(nmeshes + 1);
     FWN_CUDA_CHECK(cudaMemcpyAsync(voff, voff_h, (nmeshes + 1) * sizeof(int64_t),
                                    cudaMemcpyHostToDevice, st));
     FWN_CUDA_CHECK(cudaMemcpyAsync(foff, foff_h, (nmeshes + 1) * sizeof(int64_t),
                                    cudaMemcpyHostToDevice, st));
-    FWN_CUDA_CHECK(cudaMalloc(&e.meshes, nmeshes * sizeof(MeshInfo)));
+    e.meshes = static_cast<MeshInfo*>(engine_alloc(nmeshes * sizeof(MeshInfo), st));
     e.meshes_h = new MeshInfo[nmeshes];
-    unsigned* enc = dalloc<unsigned>(6 * nmeshes, st);
-    BuildState* bst = dalloc<BuildState>(1, st);
+    unsigned* enc = arena.take<unsigned>(6 * nmeshes);
+    BuildState* bst = arena.take<BuildState>(1);
+    StateReader reader(bst, st);
     unsigned* status = &bst->status;
     FWN_CUDA_CHECK(cudaMemsetAsync(bst, 0, sizeof(BuildState), st));
     k_init_bbox<<<grid_for(6 * nmeshes, 256), 256, 0, st>>>(enc, (int)nmeshes);
@@ -2321,19 +2368,6 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                                         e.meshes);
     FWN_CUDA_CHECK(cudaGetLastError());
 
-    struct TmpList {  // stream-ordered frees on every exit path
-        std::vector<void*> v;
-        cudaStream_t s;
-        ~TmpList() {
-            for (void* p : v) cudaFreeAsync(p, s);
-        }
-    } tmp{{}, st};
-    auto track = [&](void* p) { tmp.v.push_back(p); return p; };
-    track(voff);
-    track(foff);
-    track(enc);
-    track(bst);
-
     if (nf > 0) {
         const int n = (int)nf;
         const bool split = e.cfg.builder != FWN_BUILDER_LBVH;  // top-down (midpoint or binned)
@@ -2342,27 +2376,25 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         // a split tree at most 2n - 1 as well, ids in creation order
         const int cap = split ? 2 * n : 2 * n - 1;
         const int nint = split ? cap : std::max(n - 1, 1);  // left / right / visit entries
-        int* parent = (int*)track(dalloc<int>(cap, st));
-        int* first = (int*)track(dalloc<int>(cap, st));
-        int* last = (int*)track(dalloc<int>(cap, st));
-        int* left = (int*)track(dalloc<int>(nint, st));
-        int* right = (int*)track(dalloc<int>(nint, st));
-        int* cnt = (int*)track(dalloc<int>(n + 1, st));
-        uint8_t* flags = (uint8_t*)track(dalloc<uint8_t>(cap, st));
-        int* pos = (int*)track(dalloc<int>(cap, st));
-        int* skip = (int*)track(dalloc<int>(cap, st));
-        void* scan_tmp = track(dalloc<char>(exclusive_scan_temp_bytes(cap + 1), st));
-        int* visit = (int*)track(dalloc<int>(nint, st));
-        int* leaf_list = (int*)track(dalloc<int>(n, st));
-        int* leaf_list_len = (int*)track(dalloc<int>(1, st));
-        int* leaf_count = (int*)track(dalloc<int>(1, st));
+        int* parent = arena.take<int>(cap);
+        int* first = arena.take<int>(cap);
+        int* last = arena.take<int>(cap);
+        int* left = arena.take<int>(nint);
+        int* right = arena.take<int>(nint);
+        int* cnt = arena.take<int>(n + 1);
+        uint8_t* flags = arena.take<uint8_t>(cap);
+        int* pos = arena.take<int>(cap);
+        int* skip = arena.take<int>(cap);
+        void* scan_tmp = arena.take<char>(exclusive_scan_temp_bytes(cap + 1));
+        int* visit = split ? nullptr : arena.take<int>(nint);
+        int* leaf_list = arena.take<int>(n);
+        int* leaf_list_len = &bst->leaf_list;
         const uint64_t* keys = nullptr;
         const uint32_t* tri_of_slot = nullptr;
         int num_nodes = 0;
-        unsigned st_h = 0;
         std::vector<int> h_hist(kMaxHeight);  // internal nodes by depth or height
         // split tree: every node's depth (roots 0), the order of the level-by-level refit
-        int* depth_of = split ? (int*)track(dalloc<int>(cap, st)) : nullptr;
+        int* depth_of = split ? arena.take<int>(cap) : nullptr;
         auto check_input = [](unsigned st_h) {
             if (st_h & ST_BAD_INDEX) throw Error(FWN_INVALID_ARG, "triangle vertex index out of range");
             if (st_h & ST_NONFINITE)
@@ -2372,18 +2404,15 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         if (!split) {
             int mesh_bits = 0;
             while ((1ll << mesh_bits) < nmeshes) ++mesh_bits;
-            uint64_t* keys_a = (uint64_t*)track(dalloc<uint64_t>(n, st));
-            uint64_t* keys_b = (uint64_t*)track(dalloc<uint64_t>(n, st));
-            uint32_t* vals_a = (uint32_t*)track(dalloc<uint32_t>(n, st));
-            uint32_t* vals_b = (uint32_t*)track(dalloc<uint32_t>(n, st));
-            void* sort_tmp = track(dalloc<char>(radix_sort_temp_bytes(n, 8), st));
+            uint64_t* keys_a = arena.take<uint64_t>(n);
+            uint64_t* keys_b = arena.take<uint64_t>(n);
+            uint32_t* vals_a = arena.take<uint32_t>(n);
+            uint32_t* vals_b = arena.take<uint32_t>(n);
+            void* sort_tmp = arena.take<char>(radix_sort_temp_bytes(n, 8));
             NvtxRange trace_keys("fwn build: Morton keys + sort");
             k_tri_keys<<<grid_for(n, 256), 256, 0, st>>>(d_V, d_F, voff, foff, (int)nmeshes, nf,
                                                          e.meshes, keys_a, vals_a, status);
             FWN_CUDA_CHECK(cudaGetLastError());
-            FWN_CUDA_CHECK(cudaMemcpyAsync(&st_h, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
-            check_input(st_h);
             const bool in_b = radix_sort_u64(keys_a, vals_a, keys_b, vals_b, n,
                                              MORTON_BITS + mesh_bits, sort_tmp, st);
             keys = in_b ? keys_b : keys_a;
@@ -2401,9 +2430,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                 k_karras<<<grid_for(n - 1, 256), 256, 0, st>>>(keys, n, left, right, parent, first, last);
             }
             FWN_CUDA_CHECK(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(int), st));
-            FWN_CUDA_CHECK(cudaMemsetAsync(leaf_list_len, 0, sizeof(int), st));
             k_emit_count<<<grid_for(nn, 256), 256, 0, st>>>(n, K, keys, parent, first, last, cnt, flags,
-                                                            leaf_list, leaf_list_len);
+                                                            leaf_list, leaf_list_len,
+                                                            bst->leaf_size);
             exclusive_scan_i32(cnt, n + 1, scan_tmp, st);
             k_positions<<<grid_for(nn, 256), 256, 0, st>>>(nn, parent, first, last, flags, cnt, pos, skip);
             k_mesh_roots<<<grid_for(nmeshes, 128), 128, 0, st>>>((int)nmeshes, foff, n, parent, first,
@@ -2434,43 +2463,43 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             }
             const int nroots = (int)h_first.size();
             const int smax = n / 2 + (int)nmeshes + 1;  // active segments hold >= 2 triangles
-            uint64_t* skeys = (uint64_t*)track(dalloc<uint64_t>(n, st));
-            int* final_perm = (int*)track(dalloc<int>(n, st));
+            uint64_t* skeys = arena.take<uint64_t>(n);
+            int* final_perm = arena.take<int>(n);
             SplitSlots A, B;
             for (SplitSlots* X : {&A, &B}) {
-                X->tri = (float4*)track(dalloc<float4>(n, st));
-                X->seg = (int*)track(dalloc<int>(n, st));
+                X->tri = arena.take<float4>(n);
+                X->seg = arena.take<int>(n);
             }
             const int tiles = n / kSplitTile + 1;  // slots 0 .. n: entry n ends the last rank
             LeftRanks ranks;
-            ranks.bits = (unsigned*)track(dalloc<unsigned>(n / 32 + 1, st));
-            ranks.in_tile = (int*)track(dalloc<int>(n / 32 + 1, st));
-            ranks.tile = (int*)track(dalloc<int>(tiles, st));
-            int4* part = (int4*)track(dalloc<int4>(smax, st));
-            int2* child_next = (int2*)track(dalloc<int2>(smax, st));
-            int4* small = (int4*)track(dalloc<int4>(smax, st));
+            ranks.bits = arena.take<unsigned>(n / 32 + 1);
+            ranks.in_tile = arena.take<int>(n / 32 + 1);
+            ranks.tile = arena.take<int>(tiles);
+            int4* part = arena.take<int4>(smax);
+            int2* child_next = arena.take<int2>(smax);
+            int4* small = arena.take<int4>(smax);
             if (!h_small.empty())
                 FWN_CUDA_CHECK(cudaMemcpyAsync(small, h_small.data(), h_small.size() * sizeof(int4),
                                                cudaMemcpyHostToDevice, st));
             FWN_CUDA_CHECK(cudaMemsetAsync(depth_of, 0, (size_t)cap * sizeof(int), st));
             int* seg_a[3], *seg_b[3];  // start, end, node of this level / the next
             for (int k = 0; k < 3; ++k) {
-                seg_a[k] = (int*)track(dalloc<int>(smax, st));
-                seg_b[k] = (int*)track(dalloc<int>(smax, st));
+                seg_a[k] = arena.take<int>(smax);
+                seg_b[k] = arena.take<int>(smax);
             }
             const size_t box_words = std::max(6 * (size_t)smax, (size_t)kBoxCopies * kBoxCopyStride);
-            unsigned* box_a = (unsigned*)track(dalloc<unsigned>(box_words, st));
-            unsigned* box_b = (unsigned*)track(dalloc<unsigned>(box_words, st));
-            int* axis_of = (int*)track(dalloc<int>(smax, st));
-            float* split_of = (float*)track(dalloc<float>(smax, st));
-            int* spatial_of = (int*)track(dalloc<int>(smax, st));
-            int* bin_of = (int*)track(dalloc<int>(smax, st));
-            float* seg_box = (float*)track(dalloc<float>(6 * (size_t)smax, st));
+            unsigned* box_a = arena.take<unsigned>(box_words);
+            unsigned* box_b = arena.take<unsigned>(box_words);
+            int* axis_of = arena.take<int>(smax);
+            float* split_of = arena.take<float>(smax);
+            int* spatial_of = arena.take<int>(smax);
+            int* bin_of = arena.take<int>(smax);
+            float* seg_box = arena.take<float>(6 * (size_t)smax);
             // level-loop segments other than the roots hold more than kFinishSlots triangles each
             const int seg_bound = std::max((int)s_start.size(), n / (kFinishSlots + 1) + 1);
-            unsigned* bins = (unsigned*)track(dalloc<unsigned>((size_t)seg_bound * kSegBinWords, st));
-            int* d_mesh_seg = (int*)track(dalloc<int>(nmeshes, st));
-            int* d_root_node = (int*)track(dalloc<int>(nmeshes, st));
+            unsigned* bins = arena.take<unsigned>((size_t)seg_bound * kSegBinWords);
+            int* d_mesh_seg = arena.take<int>(nmeshes);
+            int* d_root_node = arena.take<int>(nmeshes);
             FWN_CUDA_CHECK(cudaMemcpyAsync(d_mesh_seg, mesh_seg.data(), nmeshes * sizeof(int),
                                            cudaMemcpyHostToDevice, st));
             FWN_CUDA_CHECK(cudaMemcpyAsync(d_root_node, root_node.data(), nmeshes * sizeof(int),
@@ -2512,7 +2541,6 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                            cudaMemcpyHostToDevice, st));
             SplitSlots* cur = &A;
             SplitSlots* nxt = &B;
-            StateReader reader(bst, st);
             if (nact == 0) {
                 reader.request(0);
                 check_input(reader.wait(0).status);
@@ -2578,9 +2606,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             keys = skeys;
             tri_of_slot = reinterpret_cast<const uint32_t*>(final_perm);
             FWN_CUDA_CHECK(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(int), st));
-            FWN_CUDA_CHECK(cudaMemsetAsync(leaf_list_len, 0, sizeof(int), st));
-            k_split_emit<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, first, left, flags, cnt,
-                                                                   leaf_list, leaf_list_len);
+            k_split_emit<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, first, last, left,
+                                                                   flags, cnt, leaf_list,
+                                                                   leaf_list_len, bst->leaf_size);
             exclusive_scan_i32(cnt, n + 1, scan_tmp, st);
             k_positions<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, parent, first, last,
                                                                   flags, cnt, pos, skip);
@@ -2588,33 +2616,46 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                                                        pos, skip, e.meshes);
             FWN_CUDA_CHECK(cudaGetLastError());
         }
+        // internal nodes are refitted level by level, one thread per node of a dense list (an atomic
+        // ascent would leave most lanes of its warps idle on GB300's narrow FP64 pipe): the split
+        // tree deepest first by node depth, the LBVH lowest first by node height (k_heights)
+        int* key = depth_of;
         int E = num_nodes, NL = 0;
         if (split) {  // every node is emitted, and all but the internal ones are leaves
             NL = num_nodes - std::accumulate(h_hist.begin(), h_hist.end(), 0);
         } else {
-            FWN_CUDA_CHECK(cudaMemcpyAsync(&E, cnt + n, sizeof(int), cudaMemcpyDeviceToHost, st));
-            FWN_CUDA_CHECK(cudaMemcpyAsync(&NL, leaf_list_len, sizeof(int), cudaMemcpyDeviceToHost, st));
-            FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+            key = arena.take<int>(nint);
+            if (n > 1) {
+                FWN_CUDA_CHECK(cudaMemsetAsync(visit, 0, (size_t)nint * sizeof(int), st));
+                FWN_CUDA_CHECK(cudaMemsetAsync(key, 0, (size_t)nint * sizeof(int), st));
+                k_heights<<<grid_for(n, 128), 128, 0, st>>>(leaf_list_len, leaf_list, keys, parent,
+                                                            first, last, visit, key, status);
+                k_height_hist<<<grid_for(nint, 1024), 1024, 0, st>>>(nint, keys, first, last, flags, key,
+                                                                    bst->internal, status);
+            }
+            FWN_CUDA_CHECK(cudaMemcpyAsync(&bst->emitted, cnt + n, sizeof(int),
+                                           cudaMemcpyDeviceToDevice, st));
+            FWN_CUDA_CHECK(cudaGetLastError());
+            reader.request(0);
+            const BuildState& h = reader.wait(0);
+            check_input(h.status);
+            E = h.emitted;
+            NL = h.leaf_list;
+            std::copy(h.internal, h.internal + kMaxHeight, h_hist.begin());
         }
         e.num_nodes = E;
 
         NvtxRange trace_refit("fwn build: FP64 refit, radii, records");
-        StageRec* stage = dalloc<StageRec>(E, st);
-        if (!(e.cfg.records & FWN_RECORDS_MOMENTS)) track(stage);
-        else e.stage = stage;
+        StageRec* stage = nullptr;
+        if (!(e.cfg.records & FWN_RECORDS_MOMENTS)) stage = arena.take<StageRec>(E);
+        else stage = e.stage = static_cast<StageRec*>(engine_alloc(E * sizeof(StageRec), st));
         // the refit reads the records in 16 B pairs: the pool's allocations are 256 B aligned,
         // and a build that got less stops here rather than launch misaligned vector loads
         if (reinterpret_cast<uintptr_t>(stage) % alignof(StageRec) != 0)
             throw Error(FWN_INTERNAL, "staging records are not 32 B aligned");
-        FWN_CUDA_CHECK(cudaMemsetAsync(visit, 0, (size_t)nint * sizeof(int), st));
-        FWN_CUDA_CHECK(cudaMemsetAsync(leaf_count, 0, sizeof(int), st));
         if (NL > 0) {
-            int* hist = (int*)track(dalloc<int>(kLeafSizes, st));
-            int* leaf_sorted = (int*)track(dalloc<int>(NL, st));
-            FWN_CUDA_CHECK(cudaMemsetAsync(hist, 0, kLeafSizes * sizeof(int), st));
-            k_leaf_hist<<<grid_for(NL, 256), 256, 0, st>>>(NL, leaf_list, first, last, hist);
-            k_leaf_offsets<<<1, 32, 0, st>>>(hist);
-            k_leaf_sort<<<grid_for(NL, 256), 256, 0, st>>>(NL, leaf_list, first, last, hist,
+            int* leaf_sorted = arena.take<int>(NL);
+            k_leaf_sort<<<grid_for(NL, 256), 256, 0, st>>>(NL, leaf_list, first, last, bst,
                                                           leaf_sorted);
             leaf_list = leaf_sorted;
         }
@@ -2622,27 +2663,10 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             k_refit<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_list, keys, first, last, pos,
                                                        tri_of_slot, d_V, d_F, voff, stage);
         if (NL > 0 && n > 1) {
-            // internal nodes level by level, one thread per node of a dense list (an atomic
-            // ascent would leave most lanes of its warps idle on GB300's narrow FP64 pipe): the
-            // split tree deepest first by node depth, the LBVH lowest first by node height
-            // (k_heights); the lists come from one counting sort by that key
+            // the levels' lists come from one counting sort by depth or height
             const int count = split ? num_nodes : nint;
-            int* key = depth_of;
-            if (!split) {
-                key = (int*)track(dalloc<int>(nint, st));
-                FWN_CUDA_CHECK(cudaMemsetAsync(key, 0, (size_t)nint * sizeof(int), st));
-                k_heights<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_list, keys, parent, first,
-                                                             last, visit, key, status);
-            }
-            int* offsets = (int*)track(dalloc<int>(kMaxHeight, st));
-            int* order = (int*)track(dalloc<int>(count, st));
-            if (!split) {
-                k_height_hist<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
-                                                                    bst->internal, status);
-                FWN_CUDA_CHECK(cudaMemcpyAsync(h_hist.data(), bst->internal, kMaxHeight * sizeof(int),
-                                               cudaMemcpyDeviceToHost, st));
-                FWN_CUDA_CHECK(cudaStreamSynchronize(st));
-            }
+            int* offsets = arena.take<int>(kMaxHeight);
+            int* order = arena.take<int>(count);
             std::vector<int> off(kMaxHeight + 1, 0);
             for (int h = 0; h < kMaxHeight; ++h) off[h + 1] = off[h] + h_hist[h];
             FWN_CUDA_CHECK(cudaMemcpyAsync(offsets, off.data(), kMaxHeight * sizeof(int),
@@ -2661,15 +2685,15 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             }
         }
         FWN_CUDA_CHECK(cudaGetLastError());
-        FWN_CUDA_CHECK(cudaMalloc(&e.tris, (size_t)n * sizeof(TriF32)));
-        FWN_CUDA_CHECK(cudaMalloc(&e.sorted_tri, (size_t)n * sizeof(int)));
+        e.tris = static_cast<TriF32*>(engine_alloc((size_t)n * sizeof(TriF32), st));
+        e.sorted_tri = static_cast<int*>(engine_alloc((size_t)n * sizeof(int), st));
         k_tri_records<<<grid_for(n, 256), 256, 0, st>>>(n, tri_of_slot, keys, d_V, d_F, voff,
                                                         e.tris, e.sorted_tri);
         // exact radii of the internal nodes from the triangle records: one warp per node of at
         // most kRadiusChunk triangles, chunks of the larger nodes' slot runs (the scan's last
         // entry is the chunk total)
-        int* rchunk = (int*)track(dalloc<int>(num_nodes + 1, st));
-        unsigned long long* r2bits = (unsigned long long*)track(dalloc<unsigned long long>(E, st));
+        int* rchunk = arena.take<int>(num_nodes + 1);
+        unsigned long long* r2bits = arena.take<unsigned long long>(E);
         FWN_CUDA_CHECK(cudaMemsetAsync(r2bits, 0, (size_t)E * sizeof(unsigned long long), st));
         k_radius_chunks<<<grid_for(num_nodes + 1, 256), 256, 0, st>>>(num_nodes, keys, first, last,
                                                                       flags, rchunk);
@@ -2678,42 +2702,44 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             int dev = 0, sms = 0;
             FWN_CUDA_CHECK(cudaGetDevice(&dev));
             FWN_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            int* rlist = (int*)track(dalloc<int>(num_nodes + 1, st));  // [count | list]
-            FWN_CUDA_CHECK(cudaMemsetAsync(rlist, 0, sizeof(int), st));
+            int* rlist = arena.take<int>(num_nodes);
+            int* rlen = &bst->radius_list;
             k_radius_list<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, keys, first, last,
-                                                                    flags, rlist + 1, rlist);
-            k_node_radius_small<<<sms * 8, 32 * kRadiusWarps, 0, st>>>(rlist + 1, rlist, first,
-                                                                       last, pos, stage, e.tris,
-                                                                       r2bits);
+                                                                    flags, rlist, rlen);
+            k_node_radius_small<<<sms * 8, 32 * kRadiusWarps, 0, st>>>(rlist, rlen, first, last, pos,
+                                                                       stage, e.tris, r2bits);
             k_node_radius<<<sms * 4, 256, 0, st>>>(num_nodes, rchunk, first, last, pos, stage,
                                                    e.tris, r2bits);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
-        if (e.cfg.records & FWN_RECORDS_F32) FWN_CUDA_CHECK(cudaMalloc(&e.nodes32, E * sizeof(NodeF32)));
-        if (e.cfg.records & FWN_RECORDS_F64) FWN_CUDA_CHECK(cudaMalloc(&e.nodes64, E * sizeof(NodeF64)));
-        int* node_of_pos = (int*)track(dalloc<int>(E, st));
+        if (e.cfg.records & FWN_RECORDS_F32)
+            e.nodes32 = static_cast<NodeF32*>(engine_alloc(E * sizeof(NodeF32), st));
+        if (e.cfg.records & FWN_RECORDS_F64)
+            e.nodes64 = static_cast<NodeF64*>(engine_alloc(E * sizeof(NodeF64), st));
+        int* node_of_pos = arena.take<int>(E);
         k_node_of_pos<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, flags, pos, node_of_pos);
         k_convert<<<grid_for(E, 128), 128, 0, st>>>(E, node_of_pos, keys, first, last, flags, skip,
                                                     stage, r2bits, e.nodes32, e.nodes64,
-                                                    leaf_count);
+                                                    &bst->leaf_count);
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.tuning == 7 && e.nodes32 && E > 0) {  // the structure-of-arrays layout variant
-            FWN_CUDA_CHECK(cudaMalloc(&e.soa, (size_t)E * sizeof(NodeF32)));
+            e.soa = static_cast<float4*>(engine_alloc((size_t)E * sizeof(NodeF32), st));
             k_aos_to_soa<<<grid_for(E, 256), 256, 0, st>>>(E, e.nodes32, e.soa);
             FWN_CUDA_CHECK(cudaGetLastError());
         }
-        int lc = 0;
-        FWN_CUDA_CHECK(cudaMemcpyAsync(&lc, leaf_count, sizeof(int), cudaMemcpyDeviceToHost, st));
-        FWN_CUDA_CHECK(cudaMemcpyAsync(&st_h, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-        FWN_CUDA_CHECK(cudaStreamSynchronize(st));
-        e.num_leaves = lc;
-        if (st_h & ST_REFIT_ORPHAN) throw Error(FWN_INTERNAL, "refit found an inconsistent tree");
-        if (st_h & ST_BUILD_BOUND) throw Error(FWN_INTERNAL, "split build passed its node or depth bound");
     }
     FWN_CUDA_CHECK(cudaEventRecord(ev1, st));
-    FWN_CUDA_CHECK(cudaMemcpyAsync(e.meshes_h, e.meshes, nmeshes * sizeof(MeshInfo),
-                                   cudaMemcpyDeviceToHost, st));
-    FWN_CUDA_CHECK(cudaStreamSynchronize(st));
+    const int64_t pinned = nmeshes <= StateReader::kMeshes ? nmeshes : 0;
+    if (!pinned)
+        FWN_CUDA_CHECK(cudaMemcpyAsync(e.meshes_h, e.meshes, nmeshes * sizeof(MeshInfo),
+                                       cudaMemcpyDeviceToHost, st));
+    reader.request(0, e.meshes, pinned);
+    const BuildState& done = reader.wait(0);  // the build is complete: nothing is behind it in st
+    if (pinned) std::copy(reader.meshes(0), reader.meshes(0) + nmeshes, e.meshes_h);
+    e.num_leaves = done.leaf_count;
+    if (done.status & ST_REFIT_ORPHAN) throw Error(FWN_INTERNAL, "refit found an inconsistent tree");
+    if (done.status & ST_BUILD_BOUND)
+        throw Error(FWN_INTERNAL, "split build passed its node or depth bound");
     float ms = 0.f;
     FWN_CUDA_CHECK(cudaEventElapsedTime(&ms, ev0, ev1));
     e.build_ms = ms;

@@ -62,7 +62,7 @@ template <class T> std::vector<T> to_host(const T* d, int64_t n) {
 template <class T> T* to_device(const std::vector<T>& h) {
     T* d = nullptr;
     if (h.empty()) return nullptr;
-    FWN_CUDA_CHECK(cudaMalloc(&d, h.size() * sizeof(T)));
+    d = static_cast<T*>(engine_alloc(h.size() * sizeof(T), 0));
     FWN_CUDA_CHECK(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     return d;
 }
@@ -231,7 +231,7 @@ extern "C" FWN_API fwn_status fwn_load(const char* path, fwn_handle* out) {
         e->nodes64 = to_device(n64);
         e->tris = to_device(tris);
         e->sorted_tri = to_device(sorted);
-        FWN_CUDA_CHECK(cudaMalloc(&e->meshes, (size_t)M * sizeof(MeshInfo)));
+        e->meshes = static_cast<MeshInfo*>(engine_alloc((size_t)M * sizeof(MeshInfo), 0));
         FWN_CUDA_CHECK(cudaMemcpy(e->meshes, meshes.data(), (size_t)M * sizeof(MeshInfo),
                                   cudaMemcpyHostToDevice));
         e->meshes_h = new MeshInfo[(size_t)M];

@@ -59,3 +59,46 @@ def test_coincident_centroids(torch, oracle_mod, builder, n):
     T[:, 2] = -T[:, 0] - T[:, 1]  # centroids at the origin, exactly
     T[0] += 1000
     _compare(oracle_mod, T.reshape(-1, 3), np.arange(3 * n, dtype=np.int32).reshape(-1, 3), 4, builder)
+
+
+def test_engine_memory_is_reused_safely(torch):
+    """An engine destroyed while a query on another stream still reads it: the query is right, and
+    so are the engines that take over its memory; builds from several threads, too."""
+    import threading
+    wl = W.displaced_icosphere_workload(nu=60, n_queries=400_000)
+    Q = torch.from_numpy(wl.Q).cuda()
+    w0 = fwn.FastWindingNumber(wl.V, wl.F).query(Q)[0].clone()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        eng = fwn.FastWindingNumber(wl.V, wl.F)
+        with torch.cuda.stream(side):
+            w = eng.query(Q)[0]
+        eng.close()
+        other = fwn.FastWindingNumber(wl.V * 2, wl.F)  # other values in the same memory
+        side.synchronize()
+        assert torch.equal(w, w0)
+        del other
+    out = [None] * 4
+
+    def work(i):
+        for _ in range(3):
+            out[i] = fwn.FastWindingNumber(wl.V, wl.F, builder=i % 3).info()["num_nodes"]
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert out[0] == out[3] and all(out)
+
+
+def test_build_in_capture_is_refused(torch):
+    wl = W.uv_sphere_workload(n_queries=1)
+    V, F = torch.from_numpy(wl.V).cuda(), torch.from_numpy(wl.F.astype(np.int32)).cuda()
+    x = torch.zeros(4, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        x += 1
+        with pytest.raises(fwn.WindingError):
+            fwn.FastWindingNumber(V, F)
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1, 1, 1, 1]
