@@ -415,7 +415,7 @@ struct BuildState {
     int emitted;               // nodes of the final tree (LBVH)
     int leaf_list;             // leaves listed for the refit
     int leaf_count;            // leaves among the records
-    int radius_list;           // nodes listed for k_node_radius_small
+    int radius_tiny, radius_mid, radius_chunks;  // k_radius_list's lists
     int leaf_size[kLeafSizes]; // listed leaves by triangle count
     int leaf_next[kLeafSizes]; // of those, the ones k_leaf_sort has placed
     int2 level[kMaxLevels + 1];  // active segments; nodes made before
@@ -1856,22 +1856,80 @@ __global__ void k_height_sort(int nint, const uint64_t* __restrict__ keys,
 // The far test of a node compares |q - P| with beta * r, so r must bound the distance from P to
 // every point of the node's triangles; the tightest such bound is the distance to the farthest
 // vertex (triangles are convex hulls of their vertices). Leaves compute it in leaf_moments. An
-// internal node's triangles are the contiguous run of sorted slots [first, last]. Every internal
-// node of at most kRadiusChunk triangles (all but the top few levels) takes one warp of its own
-// (a compacted list, so large and small nodes spread evenly over the warps); larger ones are
-// split into chunks of kRadiusChunk slots, one warp per chunk, whose maxima meet in an atomicMax
-// on the bit pattern (non-negative doubles order like their bits). A maximum does not depend on
-// the order, so it equals the serial one bit for bit.
-constexpr int kRadiusChunk = 2048;
+// internal node's triangles are the contiguous run of sorted slots [first, last]. Nodes of at most
+// kTinyNode triangles (most of them) take eight lanes each, nodes of at most kRadiusChunk one warp,
+// and larger ones one warp per chunk of kRadiusChunk slots, whose maxima meet in an atomicMax on
+// the bit pattern (non-negative doubles order like their bits). A maximum does not depend on the
+// order, so it equals the serial one bit for bit. A warp looks at the spheres of its groups of
+// kGroup slots first and only at the vertices of those groups that can hold the farthest one.
+// Measured, 2 million triangles: 77 us for the tiny nodes, 60 us for the next, 65 us for the larger
+// ones (a warp for each and every vertex looked at: 200 us for nodes up to 2,048 triangles, bound
+// by issue slots, and 150 us for the larger ones, bound by L2). Chunks of 2,048 slots took 27 us
+// instead of 15 in a build of 4,032 triangles, chunks of 512 took 79 us of the 2 million.
+constexpr int kRadiusChunk = 1024;
+constexpr int kTinyNode = 64;
+constexpr int kGroup = 8;
 
-// The warp's threshold after a one-pass screen, and whether a second pass is needed (some lane
-// dropped a vertex that reaches it, or the estimates left float's range).
+// What one warp looks at of the slots [s0, s1): t sees every vertex that can be the farthest from
+// P. A group's sphere (centre c, radius r about it, float) bounds its vertices: one lies at least
+// |c - P| away (c is their mean; rounding allowed for below), none farther than |c - P| + r.
+// known: a squared distance that some vertex of the node reaches (0: none known).
+// Vertices whose squared distance is 2e-5 below the largest cannot be it, in float or in double.
+__device__ __forceinline__ void screen_slots(const TriF32* __restrict__ tris,
+                                             const float4* __restrict__ groups, int s0, int s1,
+                                             const float* Pf, float known, int lane, LaneTop2& t) {
+    const int g0 = (s0 + kGroup - 1) / kGroup, g1 = s1 / kGroup;
+    float least = 0.f;  // a distance that some vertex reaches
+    if (g1 - g0 >= 8) {
+        float m = 0.f;
+        for (int g = g0 + lane; g < g1; g += 32) {
+            const float4 c = groups[g];
+            m = fmaxf(m, vertex_est(c.x, c.y, c.z, Pf));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (m > 1e-30f && m < 1e36f) {  // squares neither underflow nor overflow
+            const float d = sqrtf(m);
+            least = d - 1e-6f * (3.f * d + fabsf(Pf[0]) + fabsf(Pf[1]) + fabsf(Pf[2]));
+            least = fmaxf(least, sqrtf(known) * 0.999999f);
+        }
+    }
+    if (!(least > 0.f)) {  // few groups, or no usable bound: every vertex
+        for (int s = s0 + lane; s < s1; s += 32) t.add_slot(tris[s], Pf);
+        return;
+    }
+    const int head = g0 * kGroup - s0, tail = s1 - g1 * kGroup;  // slots outside whole groups
+    if (lane < head + tail) t.add_slot(tris[lane < head ? s0 + lane : s1 - tail + lane - head], Pf);
+    for (int b = g0; b < g1; b += 32) {
+        bool take = false;
+        if (b + lane < g1) {
+            const float4 c = groups[b + lane];
+            const float cut = least * 0.99998f - c.w;
+            take = !(cut > 0.f && vertex_est(c.x, c.y, c.z, Pf) < cut * cut * 0.99999f);
+        }
+        unsigned bal = __ballot_sync(0xffffffffu, take);
+        while (bal) {  // four groups at a time, a lane per slot
+            unsigned mine = bal;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k < (lane >> 3)) mine &= mine - 1u;
+            if (mine) t.add_slot(tris[(b + __ffs(mine) - 1) * kGroup + (lane & 7)], Pf);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bal &= bal - 1u;  // 0 stays 0
+        }
+    }
+}
+
+// The threshold of a node's LANES lanes after a one-pass screen, and whether a second pass is needed
+// (some lane dropped a vertex that reaches it, or the estimates left float's range).
+template <int LANES = 32>
 __device__ __forceinline__ bool top2_threshold(const LaneTop2& t, float& thr) {
     float m = t.m;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = LANES / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     thr = m * 0.99999f - 1e-37f;
-    return __any_sync(0xffffffffu, !(m < INFINITY) || !(t.dropped < thr));
+    const unsigned bal = __ballot_sync(0xffffffffu, !(m < INFINITY) || !(t.dropped < thr));
+    return LANES == 32 ? bal != 0u : (bal >> (threadIdx.x & 31 & ~(LANES - 1)) & ((1u << (LANES & 31)) - 1u)) != 0u;
 }
 
 // Largest vertex_r2 over slots [s0, s1), one warp: a one-pass float screen (LaneTop2), then the
@@ -1880,11 +1938,12 @@ __device__ __forceinline__ bool top2_threshold(const LaneTop2& t, float& thr) {
 // all, or near float's underflow or overflow, where every vertex is taken). The vertex with the
 // largest exact term always qualifies, so the result is the plain FP64 maximum bit for bit, at a
 // few FP64 terms per run instead of three per triangle.
-__device__ __forceinline__ double slots_r2(const TriF32* __restrict__ tris, int s0, int s1,
-                                           const double* P, int lane) {
+__device__ __forceinline__ double slots_r2(const TriF32* __restrict__ tris,
+                                           const float4* __restrict__ groups, int s0, int s1,
+                                           const double* P, float known, int lane) {
     const float Pf[3] = {d2f(P[0]), d2f(P[1]), d2f(P[2])};
     LaneTop2 t;
-    for (int s = s0 + lane; s < s1; s += 32) t.add_slot(tris[s], Pf);
+    screen_slots(tris, groups, s0, s1, Pf, known, lane, t);
     float thr;
     double r2 = 0.0;
     if (top2_threshold(t, thr)) {
@@ -1912,38 +1971,42 @@ __device__ __forceinline__ bool internal_emitted(const uint64_t* __restrict__ ke
     return (fl & 1) && !(fl & 2) && !is_cross(keys, first, last, u);
 }
 
-// chunks[u] for the nodes u < num_nodes (0 unless an emitted single-mesh internal node of more than
-// kRadiusChunk triangles); chunks[num_nodes] = 0 becomes the total after the exclusive scan.
-__global__ void k_radius_chunks(int num_nodes, const uint64_t* __restrict__ keys,
-                                const int* __restrict__ first, const int* __restrict__ last,
-                                const uint8_t* __restrict__ flags, int* __restrict__ chunks) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u > num_nodes) return;
-    chunks[u] = (u < num_nodes && internal_emitted(keys, first, last, flags, u) &&
-                 last[u] - first[u] + 1 > kRadiusChunk)
-                    ? (last[u] - first[u] + kRadiusChunk) / kRadiusChunk
-                    : 0;
-}
-
-// The internal nodes of at most kRadiusChunk triangles, in any order (list[0 .. *count)).
+// The internal nodes, in any order: those of at most kTinyNode triangles from the front of
+// list[0 .. num_nodes), those of at most kRadiusChunk from its end, and the larger ones' chunks
+// {node, first slot}, as many as fit into the bound of kMaxHeight levels.
 __global__ void k_radius_list(int num_nodes, const uint64_t* __restrict__ keys,
                               const int* __restrict__ first, const int* __restrict__ last,
-                              const uint8_t* __restrict__ flags, int* __restrict__ list,
-                              int* __restrict__ count) {
+                              const uint8_t* __restrict__ flags, BuildState* __restrict__ bst,
+                              int* __restrict__ list, int2* __restrict__ chunks, int max_chunks) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool pred = u < num_nodes && internal_emitted(keys, first, last, flags, u) &&
-                      last[u] - first[u] + 1 <= kRadiusChunk;
-    const int at = block_append(count, pred);
-    if (at >= 0) list[at] = u;
+    const bool node = u < num_nodes && internal_emitted(keys, first, last, flags, u);
+    const int f = node ? first[u] : 0, size = node ? last[u] - f + 1 : 0;
+    const int tiny = block_append(&bst->radius_tiny, node && size <= kTinyNode);
+    if (tiny >= 0) list[tiny] = u;
+    const int mid = block_append(&bst->radius_mid, node && size > kTinyNode && size <= kRadiusChunk);
+    if (mid >= 0) list[num_nodes - 1 - mid] = u;
+    // the warp writes each larger node's chunks together
+    const int nc = size > kRadiusChunk ? (size + kRadiusChunk - 1) / kRadiusChunk : 0;
+    int at = 0;
+    if (nc) {
+        at = atomicAdd(&bst->radius_chunks, nc);
+        if (at + nc > max_chunks) atomicOr(&bst->status, ST_BUILD_BOUND);
+    }
+    for (unsigned bal = __ballot_sync(0xffffffffu, nc > 0); bal; bal &= bal - 1u) {
+        const int k = __ffs(bal) - 1;
+        const int wn = __shfl_sync(0xffffffffu, nc, k), wa = __shfl_sync(0xffffffffu, at, k);
+        const int wu = __shfl_sync(0xffffffffu, u, k), wf = __shfl_sync(0xffffffffu, f, k);
+        for (int c = threadIdx.x & 31; c < wn && wa + c < max_chunks; c += 32)
+            chunks[wa + c] = make_int2(wu, wf + c * kRadiusChunk);
+    }
 }
 
-// One warp per listed node (grid-stride), all lanes on its slot run. The float screen runs per
-// node in one pass (LaneTop2; a second pass only on ties); the vertices that pass it (a few per
-// node) queue in the warp's shared buffer across the
-// warp's nodes and get their exact FP64 terms 32 at a time, one per lane, so the FP64 pipe (2
+// LANES lanes per listed node (grid-stride). The float screen runs per node in one pass (LaneTop2; a
+// second pass only on ties); the vertices that pass it (a few per node) queue in the warp's shared
+// buffer across the warp's nodes and get their exact FP64 terms 32 at a time, one per lane, so the FP64 pipe (2
 // operations per SM per cycle on GB300, whatever the number of active lanes) sees full warps;
 // each term goes to its node's maximum by atomicMax on the bit pattern (r2bits starts at 0).
-constexpr int kRadiusWarps = 8;      // warps per block of k_node_radius_small
+constexpr int kRadiusWarps = 8;      // warps per block of k_node_radius_listed
 constexpr int kRadiusQueue = 64;     // queued vertices per warp (< 32 left + 32 added)
 
 struct RadiusQueue {
@@ -1964,11 +2027,15 @@ __device__ __forceinline__ void radius_flush(RadiusQueue& q, int count,
     __syncwarp();
 }
 
+template <int LANES>
 __global__ void __launch_bounds__(32 * kRadiusWarps)
-k_node_radius_small(const int* __restrict__ list, const int* __restrict__ count,
-                    const int* __restrict__ first, const int* __restrict__ last,
-                    const int* __restrict__ pos, const StageRec* __restrict__ stage,
-                    const TriF32* __restrict__ tris, unsigned long long* __restrict__ r2bits) {
+k_node_radius_listed(const int* __restrict__ list, int step, const int* __restrict__ count,
+                     const int* __restrict__ first, const int* __restrict__ last,
+                     const int* __restrict__ pos, const StageRec* __restrict__ stage,
+                     const TriF32* __restrict__ tris, const float4* __restrict__ groups,
+                     unsigned long long* __restrict__ r2bits) {
+    static_assert(LANES == 8 || LANES == 32, "a node's lanes: eight or the warp");
+    constexpr int kNodes = 32 / LANES;  // nodes a warp has in hand
     __shared__ RadiusQueue queues[kRadiusWarps];
     RadiusQueue& q = queues[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -1999,24 +2066,33 @@ k_node_radius_small(const int* __restrict__ list, const int* __restrict__ count,
             queued -= 32;
         }  // queued < 32 here: the next step adds at most 32 (< kRadiusQueue)
     };
-    for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < total; w += nwarps) {
-        const int v = list[w];
-        const int i = pos[v];
-        const int s0 = first[v], s1 = last[v] + 1;
+    const int sub = lane % LANES;
+    for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kNodes; w < total;
+         w += nwarps * kNodes) {
+        const bool on = w + lane / LANES < total;
+        const int v = on ? list[step * (w + lane / LANES)] : 0;
+        const int i = on ? pos[v] : 0;
+        const int s0 = on ? first[v] : 0, s1 = on ? last[v] + 1 : 0;
         const float Pf[3] = {d2f(stage[i].P[0]), d2f(stage[i].P[1]), d2f(stage[i].P[2])};
         LaneTop2 t;
-        for (int s = s0 + lane; s < s1; s += 32) t.add_slot(tris[s], Pf);
+        if (LANES == 32) screen_slots(tris, groups, s0, s1, Pf, 0.f, lane, t);
+        else
+            for (int s = s0 + sub; s < s1; s += LANES) t.add_slot(tris[s], Pf);
         float thr;
-        if (!top2_threshold(t, thr)) {  // the two kept per lane hold every candidate
-            enqueue(t.e0 >= thr, t.x0, t.y0, t.z0, i);
-            enqueue(t.e1 >= thr, t.x1, t.y1, t.z1, i);
-            continue;
-        }
+        const bool again = top2_threshold<LANES>(t, thr);
+        // the two kept per lane hold every candidate
+        const bool keep = on && !again;
+        enqueue(keep && t.e0 >= thr, t.x0, t.y0, t.z0, i);
+        enqueue(keep && t.e1 >= thr, t.x1, t.y1, t.z1, i);
+        if (!__any_sync(0xffffffffu, on && again)) continue;
         const bool all = !(thr < INFINITY);
-        for (int base = s0; base < s1; base += 32) {  // second pass, warp-uniform trip count
-            const int s = base + lane;
+        int rounds = on && again ? (s1 - s0 + LANES - 1) / LANES : 0;
+        rounds = __reduce_max_sync(0xffffffffu, rounds);
+        for (int r = 0; r < rounds; ++r) {  // second pass, warp-uniform trip count
+            const int s = s0 + r * LANES + sub;
+            const bool in = again && s < s1;
             float vx[3] = {0.f, 0.f, 0.f}, vy[3] = {0.f, 0.f, 0.f}, vz[3] = {0.f, 0.f, 0.f};
-            if (s < s1) {
+            if (in) {
                 const float4 t0 = tris[s].t0, t1 = tris[s].t1, t2 = tris[s].t2;
                 vx[0] = t0.x; vy[0] = t0.y; vz[0] = t0.z;
                 vx[1] = t0.w; vy[1] = t1.x; vz[1] = t1.y;
@@ -2024,34 +2100,29 @@ k_node_radius_small(const int* __restrict__ list, const int* __restrict__ count,
             }
 #pragma unroll
             for (int j = 0; j < 3; ++j)
-                enqueue(s < s1 && (all || vertex_est(vx[j], vy[j], vz[j], Pf) >= thr), vx[j], vy[j],
-                        vz[j], i);
+                enqueue(in && (all || vertex_est(vx[j], vy[j], vz[j], Pf) >= thr), vx[j], vy[j], vz[j], i);
         }
     }
     if (queued > 0) radius_flush(q, queued, stage, r2bits, lane);
 }
 
-// Grid-stride over the chunks: chunk c belongs to the last node u with off[u] <= c.
-__global__ void k_node_radius(int num_nodes, const int* __restrict__ off,
-                              const int* __restrict__ first, const int* __restrict__ last,
+// The larger nodes, one warp per chunk (grid-stride).
+__global__ void k_node_radius(const int2* __restrict__ chunks, const int* __restrict__ count,
+                              int max_chunks, const int* __restrict__ last,
                               const int* __restrict__ pos, const StageRec* __restrict__ stage,
-                              const TriF32* __restrict__ tris,
+                              const TriF32* __restrict__ tris, const float4* __restrict__ groups,
                               unsigned long long* __restrict__ r2bits) {
     const int lane = threadIdx.x & 31;
-    const int total = off[num_nodes];
+    const int total = min(*count, max_chunks);
     const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
     for (int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < total; c += nwarps) {
-        int lo = 0, hi = num_nodes - 1;  // off[num_nodes] = total > c
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (off[mid] <= c) lo = mid; else hi = mid - 1;
-        }
-        const int u = lo;
-        const int s0 = first[u] + (c - off[u]) * kRadiusChunk;
-        const int s1 = min(last[u] + 1, s0 + kRadiusChunk);
-        const int i = pos[u];
+        const int2 at = chunks[c];
+        const int s0 = at.y, s1 = min(last[at.x] + 1, s0 + kRadiusChunk);
+        const int i = pos[at.x];
         const double P[3] = {stage[i].P[0], stage[i].P[1], stage[i].P[2]};
-        const double r2 = slots_r2(tris, s0, s1, P, lane);
+        // what the node's other chunks have found so far: less only if one of them just raised it
+        const float known = d2f(__longlong_as_double((long long)__ldcg(&r2bits[i])));
+        const double r2 = slots_r2(tris, groups, s0, s1, P, known, lane);
         if (lane == 0) atomicMax(&r2bits[i], (unsigned long long)__double_as_longlong(r2));
     }
 }
@@ -2185,9 +2256,10 @@ __global__ void k_aos_to_soa(int64_t num_nodes, const NodeF32* __restrict__ n32,
 __global__ void k_tri_records(int n, const uint32_t* __restrict__ tri_of_slot,
                               const uint64_t* __restrict__ keys, const float* __restrict__ V,
                               const int32_t* __restrict__ F, const int64_t* __restrict__ voff,
-                              TriF32* __restrict__ tris, int* __restrict__ sorted_tri) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
+                              TriF32* __restrict__ tris, int* __restrict__ sorted_tri,
+                              float4* __restrict__ groups) {
+    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = min(at, n - 1);  // (the lanes past the end stay for the group's reductions)
     const int64_t t = tri_of_slot[s];
     const int m = (int)(keys[s] >> MORTON_BITS);
     float v[3][3];
@@ -2197,6 +2269,22 @@ __global__ void k_tri_records(int n, const uint32_t* __restrict__ tri_of_slot,
         v[j][1] = V[3 * vi + 1];
         v[j][2] = V[3 * vi + 2];
     }
+    // the sphere of the group's kGroup slots about the mean of their vertices (screen_slots)
+    float gc[3], g2 = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        gc[a] = (v[0][a] + v[1][a]) + v[2][a];
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) gc[a] += __shfl_xor_sync(0xffffffffu, gc[a], o);
+        gc[a] *= 1.0f / (3 * kGroup);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) g2 = fmaxf(g2, vertex_est(v[j][0], v[j][1], v[j][2], gc));
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1) g2 = fmaxf(g2, __shfl_xor_sync(0xffffffffu, g2, o));
+    if (at >= n) return;
+    if (s % kGroup == 0)
+        groups[s / kGroup] = make_float4(gc[0], gc[1], gc[2], sqrtf(g2) * 1.000002f);
     float c[3];
     for (int a = 0; a < 3; ++a) c[a] = ((v[0][a] + v[1][a]) + v[2][a]) / 3.0f;
     float rt = 0.f;
@@ -2687,29 +2775,33 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         FWN_CUDA_CHECK(cudaGetLastError());
         e.tris = static_cast<TriF32*>(engine_alloc((size_t)n * sizeof(TriF32), st));
         e.sorted_tri = static_cast<int*>(engine_alloc((size_t)n * sizeof(int), st));
+        float4* groups = arena.take<float4>((n + kGroup - 1) / kGroup);
         k_tri_records<<<grid_for(n, 256), 256, 0, st>>>(n, tri_of_slot, keys, d_V, d_F, voff,
-                                                        e.tris, e.sorted_tri);
-        // exact radii of the internal nodes from the triangle records: one warp per node of at
-        // most kRadiusChunk triangles, chunks of the larger nodes' slot runs (the scan's last
-        // entry is the chunk total)
-        int* rchunk = arena.take<int>(num_nodes + 1);
+                                                        e.tris, e.sorted_tri, groups);
+        // exact radii of the internal nodes from the triangle records
         unsigned long long* r2bits = arena.take<unsigned long long>(E);
         FWN_CUDA_CHECK(cudaMemsetAsync(r2bits, 0, (size_t)E * sizeof(unsigned long long), st));
-        k_radius_chunks<<<grid_for(num_nodes + 1, 256), 256, 0, st>>>(num_nodes, keys, first, last,
-                                                                      flags, rchunk);
-        exclusive_scan_i32(rchunk, num_nodes + 1, scan_tmp, st);
         if (n > 1) {
             int dev = 0, sms = 0;
             FWN_CUDA_CHECK(cudaGetDevice(&dev));
             FWN_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             int* rlist = arena.take<int>(num_nodes);
-            int* rlen = &bst->radius_list;
+            // a level's larger nodes are n / kRadiusChunk at most, with as many whole chunks
+            const int max_chunks = 2 * kMaxHeight * (n / kRadiusChunk);
+            int2* chunks = arena.take<int2>(max_chunks);
             k_radius_list<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, keys, first, last,
-                                                                    flags, rlist, rlen);
-            k_node_radius_small<<<sms * 8, 32 * kRadiusWarps, 0, st>>>(rlist, rlen, first, last, pos,
-                                                                       stage, e.tris, r2bits);
-            k_node_radius<<<sms * 4, 256, 0, st>>>(num_nodes, rchunk, first, last, pos, stage,
-                                                   e.tris, r2bits);
+                                                                    flags, bst, rlist, chunks,
+                                                                    max_chunks);
+            const int threads = 32 * kRadiusWarps;
+            k_node_radius_listed<8><<<sms * 8, threads, 0, st>>>(
+                rlist, 1, &bst->radius_tiny, first, last, pos, stage, e.tris, groups, r2bits);
+            if (n > kTinyNode)
+                k_node_radius_listed<32><<<sms * 8, threads, 0, st>>>(
+                    rlist + num_nodes - 1, -1, &bst->radius_mid, first, last, pos, stage, e.tris,
+                    groups, r2bits);
+            if (n > kRadiusChunk)
+                k_node_radius<<<sms * 8, 256, 0, st>>>(chunks, &bst->radius_chunks, max_chunks, last,
+                                                       pos, stage, e.tris, groups, r2bits);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.records & FWN_RECORDS_F32)

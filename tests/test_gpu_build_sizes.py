@@ -102,3 +102,15 @@ def test_build_in_capture_is_refused(torch):
     g.replay()
     torch.cuda.synchronize()
     assert x.tolist() == [1, 1, 1, 1]
+
+
+@pytest.mark.parametrize("builder", [fwn.BUILDER_LBVH, fwn.BUILDER_SPLIT])
+@pytest.mark.parametrize("scale,shift", [(1e-20, 0), (1e-12, 0), (1e17, 0), (1.0, 3e4), (1e-3, 30.0)])
+def test_radii_at_scales(torch, oracle_mod, builder, scale, shift):
+    """Squared lengths at both ends of float (every vertex is looked at there), and meshes far from
+    the origin, where the group spheres' centres round coarsely; a sphere (every vertex of the root
+    is a candidate) with some long triangles."""
+    wl = W.displaced_icosphere_workload(nu=20, n_queries=1)
+    V, F = wl.V.astype(np.float64), wl.F.copy()
+    F[::97, 1] = F[0, 0]
+    _compare(oracle_mod, ((V + shift) * scale).astype(np.float32), F, 4, builder)
