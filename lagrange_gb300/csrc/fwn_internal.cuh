@@ -182,17 +182,18 @@ struct Scratch {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Radix sort (radix_sort.cu): stable LSD sort of (key, value) pairs, 8-bit digits.
-// Sorts keys_a/vals_a using keys_b/vals_b as ping-pong buffers; returns true when the result
-// ended in the *_b buffers. temp holds 256 digit counts per tile of kSortTileKeys keys, plus the
-// 256 digit totals (radix_sort_temp_bytes).
+// Radix sort (radix_sort.cu): stable LSD sort of n keys by their bits [begin_bit, end_bit), 8-bit
+// digits; the bits from end_bit up are zero. The values are the keys' places before the sort.
+// Sorts keys_a using keys_b as the other buffer; returns true when the keys and values ended in
+// the *_b buffers. temp holds 256 digit counts per tile of kSortTileKeys keys (for few tiles, of
+// every pass), plus the 256 digit totals (radix_sort_temp_bytes).
 // ---------------------------------------------------------------------------------------------
 constexpr int kSortTileKeys = 2048;  // keys per sort tile: 256 threads x 8 keys
 size_t radix_sort_temp_bytes(int64_t n, int key_bytes);
 bool radix_sort_u32(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b,
-                    int64_t n, int key_bits, void* temp, cudaStream_t stream);
+                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream);
 bool radix_sort_u64(uint64_t* keys_a, uint32_t* vals_a, uint64_t* keys_b, uint32_t* vals_b,
-                    int64_t n, int key_bits, void* temp, cudaStream_t stream);
+                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream);
 
 // Exclusive scan of n int32 values in place (radix_sort.cu).
 size_t exclusive_scan_temp_bytes(int64_t n);
@@ -275,6 +276,7 @@ QueryArgs resolve_query_args(const Engine& e, const fwn_query_opts* opts);
 struct ForestKeys {
     int mesh_bits = 0, hilbert_bits = 30, key_bits = 30;
     bool narrow = true;
+    int64_t max_queries = 0;  // of one mesh
 };
 ForestKeys forest_keys(int64_t nmeshes, const int64_t* query_offsets);
 

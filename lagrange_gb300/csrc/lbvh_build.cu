@@ -146,8 +146,7 @@ __global__ void k_mesh_info(const unsigned* __restrict__ enc, const int64_t* __r
 __global__ void k_tri_keys(const float* __restrict__ V, const int32_t* __restrict__ F,
                            const int64_t* __restrict__ voff, const int64_t* __restrict__ foff,
                            int nmeshes, int64_t nf, const MeshInfo* __restrict__ mi,
-                           uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                           unsigned* __restrict__ status) {
+                           uint64_t* __restrict__ keys, unsigned* __restrict__ status) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nf) return;
     const int m = find_mesh(foff, nmeshes, t);
@@ -181,7 +180,6 @@ __global__ void k_tri_keys(const float* __restrict__ V, const int32_t* __restric
                     (spread3(quantize10(c[1], M.lo[1], M.inv_ext[1])) << 1) |
                     spread3(quantize10(c[2], M.lo[2], M.inv_ext[2]));
     keys[t] = ((uint64_t)m << MORTON_BITS) | code;
-    vals[t] = (uint32_t)t;
 }
 
 // ---- K3: Karras hierarchy ---------------------------------------------------------------------
@@ -2499,10 +2497,10 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             void* sort_tmp = arena.take<char>(radix_sort_temp_bytes(n, 8));
             NvtxRange trace_keys("fwn build: Morton keys + sort");
             k_tri_keys<<<grid_for(n, 256), 256, 0, st>>>(d_V, d_F, voff, foff, (int)nmeshes, nf,
-                                                         e.meshes, keys_a, vals_a, status);
+                                                         e.meshes, keys_a, status);
             FWN_CUDA_CHECK(cudaGetLastError());
             const bool in_b = radix_sort_u64(keys_a, vals_a, keys_b, vals_b, n,
-                                             MORTON_BITS + mesh_bits, sort_tmp, st);
+                                             0, MORTON_BITS + mesh_bits, sort_tmp, st);
             keys = in_b ? keys_b : keys_a;
             tri_of_slot = in_b ? vals_b : vals_a;
 

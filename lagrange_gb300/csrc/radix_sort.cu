@@ -6,6 +6,10 @@
 //   downsweep : tile keys ranked stably within each warp (lanes holding the same digit found
 //               with one ballot per digit bit), scattered into shared memory in digit order,
 //               then written out with runs of consecutive addresses
+// Up to kFewTiles tiles one launch per pass, and one before the first: there a pass is the latency
+// of its launches, so a block adds up the digits' tile counts itself, and counts what it writes for
+// the next pass. (A pass over 100,000 keys takes 12 us, 17 with three launches; the two meet at about
+// 262,000 keys, where each block adds up 128 tiles.)
 // Stability comes from the warp-striped load order (warp, round, lane) = input order.
 // Used for the triangle Morton keys (u64: mesh id above 30 Morton bits) and the query keys.
 #include "fwn_internal.cuh"
@@ -125,11 +129,42 @@ k_scan_digits(int* __restrict__ hist, int nblocks, int* __restrict__ digit_total
     if (tid == 0) digit_totals[blockIdx.x] = carry_s;
 }
 
+// Few tiles: the first pass's tile histograms (tile-major, [tile][digit]), and zeros for those of
+// the passes after it.
+constexpr int kFewTiles = 128;
 template <class K>
+__global__ void __launch_bounds__(SORT_THREADS)
+k_few_hist(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hist, int passes) {
+    constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
+    __shared__ int h[RADIX];
+    const int tid = threadIdx.x;
+    const int64_t base = (int64_t)blockIdx.x * TILE;
+    K k[KPT];
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const int64_t idx = base + (int64_t)j * SORT_THREADS + tid;
+        k[j] = idx < n ? keys[idx] : (K)0;
+    }
+    h[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < KPT; ++j)
+        if (base + (int64_t)j * SORT_THREADS + tid < n)
+            atomicAdd(&h[(unsigned)(k[j] >> shift) & (RADIX - 1)], 1);
+    __syncthreads();
+    const int at = blockIdx.x * RADIX + tid;
+    hist[at] = h[tid];
+    for (int p = 1; p < passes; ++p) hist[p * (int)gridDim.x * RADIX + at] = 0;
+}
+
+// hist: of this pass, digit-major and scanned along the tiles; with FEW, the counts [tile][digit].
+// hist_next (FEW): the next pass's, or null.
+template <class K, bool FEW>
 __global__ void __launch_bounds__(SORT_THREADS)
 k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
             K* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n, int shift,
-            const int* __restrict__ hist, const int* __restrict__ digit_totals, int nblocks) {
+            const int* __restrict__ hist, const int* __restrict__ digit_totals,
+            int* __restrict__ hist_next, int nblocks) {
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ K skeys[TILE];
     __shared__ uint32_t svals[TILE];
@@ -153,13 +188,28 @@ k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
         int64_t idx = base + (int64_t)w * (KPT * 32) + j * 32 + lane;
         bool valid = idx < n;
         k[j] = valid ? keys_in[idx] : (K)0;
-        v[j] = valid ? vals_in[idx] : 0u;
+        v[j] = !valid ? 0u : vals_in ? vals_in[idx] : (uint32_t)idx;
     }
     // Global base of each digit for this tile: exclusive scan of the digit totals plus this
     // tile's exclusive offset within the digit.
     {
-        const int tile_off = hist[(int64_t)tid * nblocks + blockIdx.x];
-        int dt = digit_totals[tid];
+        int tile_off = 0, dt = 0;
+        if (FEW) {
+            constexpr int kAhead = 16;  // loads in flight
+            for (int b = 0; b < nblocks; b += kAhead) {
+                int x[kAhead];
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) x[j] = b + j < nblocks ? hist[(b + j) * RADIX + tid] : 0;
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) {
+                    dt += x[j];
+                    tile_off += b + j < (int)blockIdx.x ? x[j] : 0;
+                }
+            }
+        } else {
+            tile_off = hist[(int64_t)tid * nblocks + blockIdx.x];
+            dt = digit_totals[tid];
+        }
         int ex = block_exclusive_scan_256(dt, warp_tot);
         gbase[tid] = ex + tile_off;
     }
@@ -221,29 +271,47 @@ k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
         int64_t out = (int64_t)gbase[d] + (i - tile_start[d]);
         keys_out[out] = kk;
         vals_out[out] = svals[i];
+        if (FEW && hist_next)
+            atomicAdd(&hist_next[(int)(out / TILE) * RADIX + ((unsigned)(kk >> (shift + RADIX_BITS)) & (RADIX - 1))], 1);
     }
 }
 
 template <class K>
-bool radix_sort_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, int64_t n, int key_bits,
-                     void* temp, cudaStream_t stream) {
-    if (n <= 1 || key_bits <= 0) return false;
+bool radix_sort_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, int64_t n, int begin_bit,
+                     int end_bit, void* temp, cudaStream_t stream) {
+    if (n <= 1 || end_bit <= begin_bit) {
+        if (n == 1) FWN_CUDA_CHECK(cudaMemsetAsync(va, 0, sizeof(uint32_t), stream));
+        return false;
+    }
     constexpr int TILE = TileCfg<K>::TILE;
     const int nblocks = (int)((n + TILE - 1) / TILE);
     int* hist = static_cast<int*>(temp);
     int* totals = hist + (int64_t)RADIX * nblocks;
     K* ks = ka;
     K* kd = kb;
-    uint32_t* vs = va;
+    const uint32_t* vs = nullptr;  // the first pass makes the values: the keys' places
     uint32_t* vd = vb;
     bool in_b = false;
-    for (int shift = 0; shift < key_bits; shift += RADIX_BITS) {
-        k_upsweep<K><<<nblocks, SORT_THREADS, 0, stream>>>(ks, n, shift, hist, nblocks);
-        k_scan_digits<<<RADIX, 1024, 0, stream>>>(hist, nblocks, totals);
-        k_downsweep<K><<<nblocks, SORT_THREADS, 0, stream>>>(ks, vs, kd, vd, n, shift, hist,
-                                                              totals, nblocks);
+    const bool few = nblocks <= kFewTiles;
+    if (few)
+        k_few_hist<K><<<nblocks, SORT_THREADS, 0, stream>>>(
+            ks, n, begin_bit, hist, (end_bit - begin_bit + RADIX_BITS - 1) / RADIX_BITS);
+    for (int shift = begin_bit; shift < end_bit; shift += RADIX_BITS) {
+        if (few) {
+            int* next = hist + (int64_t)RADIX * nblocks;
+            k_downsweep<K, true><<<nblocks, SORT_THREADS, 0, stream>>>(
+                ks, vs, kd, vd, n, shift, hist, nullptr, shift + RADIX_BITS < end_bit ? next : nullptr,
+                nblocks);
+            hist = next;
+        } else {
+            k_upsweep<K><<<nblocks, SORT_THREADS, 0, stream>>>(ks, n, shift, hist, nblocks);
+            k_scan_digits<<<RADIX, 1024, 0, stream>>>(hist, nblocks, totals);
+            k_downsweep<K, false><<<nblocks, SORT_THREADS, 0, stream>>>(ks, vs, kd, vd, n, shift, hist,
+                                                                        totals, nullptr, nblocks);
+        }
         std::swap(ks, kd);
-        std::swap(vs, vd);
+        vs = vd;
+        vd = in_b ? vb : va;
         in_b = !in_b;
     }
     FWN_CUDA_CHECK(cudaGetLastError());
@@ -354,17 +422,19 @@ k_scan_tiles(int* __restrict__ data, int64_t n, const int* __restrict__ sums) {
 size_t radix_sort_temp_bytes(int64_t n, int key_bytes) {
     const int tile = key_bytes == 8 ? TileCfg<uint64_t>::TILE : TileCfg<uint32_t>::TILE;
     const int64_t nblocks = (n + tile - 1) / tile;
-    return (size_t)(RADIX * nblocks + RADIX) * sizeof(int) + 256;
+    // few tiles: a histogram for each pass (of 8 key_bytes bits)
+    const int64_t hists = nblocks <= kFewTiles ? key_bytes : 1;
+    return (size_t)(RADIX * nblocks * hists + RADIX) * sizeof(int) + 256;
 }
 
 bool radix_sort_u32(uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, int64_t n,
-                    int key_bits, void* temp, cudaStream_t stream) {
-    return radix_sort_impl<uint32_t>(ka, va, kb, vb, n, key_bits, temp, stream);
+                    int begin_bit, int end_bit, void* temp, cudaStream_t stream) {
+    return radix_sort_impl<uint32_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream);
 }
 
 bool radix_sort_u64(uint64_t* ka, uint32_t* va, uint64_t* kb, uint32_t* vb, int64_t n,
-                    int key_bits, void* temp, cudaStream_t stream) {
-    return radix_sort_impl<uint64_t>(ka, va, kb, vb, n, key_bits, temp, stream);
+                    int begin_bit, int end_bit, void* temp, cudaStream_t stream) {
+    return radix_sort_impl<uint64_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream);
 }
 
 size_t exclusive_scan_temp_bytes(int64_t n) {
