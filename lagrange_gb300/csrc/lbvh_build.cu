@@ -380,7 +380,7 @@ constexpr int kSpatialLevels = 96;
 // Segments of at most kFinishSlots triangles leave the level loop: one block each finishes their
 // subtrees in shared memory (k_split_finish), with the same splits.
 constexpr int kFinishSlots = 1024;
-constexpr int kFinishThreads = 512;
+constexpr int kFinishThreads = 384;
 // Segments of the level loop (more than kFinishSlots triangles) split at a binned plane: kSplitBins
 // bins per axis over the centroid box, bin(x) = min((int)((x - lo) / ext * 16), 15) in float, and
 // the plane with the least nL * dL + nR * dR (d = squared diagonal of a side's centroid bounds, in
@@ -1094,15 +1094,18 @@ __global__ void k_split_scatter(int64_t n, const BuildState* __restrict__ bst, L
 
 // A small segment in shared memory. Sub-segments are named by their first position, so a
 // split names its children itself (b and mid); the slots carry their original local index, and
-// centroids stay where they were loaded.
+// centroids stay where they were loaded. Active segments hold two slots or more, so the tables of
+// segments have an entry per two positions: 46 KB, four blocks per SM. A step is a chain of
+// barriers, so what counts is the blocks in flight (2 million triangles, 2,900 blocks: 229 us with
+// four of 384 threads, 266 with three of 512 and 64 KB).
 struct FinishShared {
     float c[3][kFinishSlots];              // centroid of each original local slot
     int perm[kFinishSlots];                // triangle of each original local slot
     unsigned short orig[2][kFinishSlots];  // original local slot at each position
     short sid[2][kFinishSlots];            // first position of the position's segment (-1: leaf)
-    short send[2][kFinishSlots];           // end of the segment that starts at a position
-    int snode[2][kFinishSlots];            // node of the segment that starts at a position
-    unsigned box[6][kFinishSlots];         // centroid box of the segment that starts there
+    short send[2][kFinishSlots / 2];       // end of the segment that starts at a position
+    int snode[2][kFinishSlots / 2];        // node of the segment that starts at a position
+    unsigned box[6][kFinishSlots / 2];     // centroid box of the segment that starts there
     int scan[kFinishSlots + 1];
     int wsum[kFinishThreads / 32];
     int ns[2], rank, node_base;
@@ -1148,7 +1151,7 @@ __device__ void block_exclusive_scan(int* a, int count, int* wsum) {
 // an even depth and in B for an odd one (the level that made the segment wrote them there, and
 // later levels write only other segments' ranges). Each step's node ids are one allocation after
 // the level loop's nodes.
-__global__ void __launch_bounds__(kFinishThreads) k_split_finish(
+__global__ void __launch_bounds__(kFinishThreads, 4) k_split_finish(
     const int4* __restrict__ small, SplitSlots A, SplitSlots B, int K, BuildState* __restrict__ bst,
     int level_nodes, int cap, int* __restrict__ nfirst, int* __restrict__ nlast,
     int* __restrict__ nparent, int* __restrict__ nleft, int* __restrict__ nright,
@@ -1205,8 +1208,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
                     const unsigned ev = enc_float(S.c[a][o]);
                     const unsigned lo = __reduce_min_sync(peers, ev), hi = __reduce_max_sync(peers, ev);
                     if (leader) {
-                        atomicMin(&S.box[a][key], lo);
-                        atomicMax(&S.box[3 + a][key], hi);
+                        atomicMin(&S.box[a][key >> 1], lo);
+                        atomicMax(&S.box[3 + a][key >> 1], hi);
                     }
                 }
             }
@@ -1230,8 +1233,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
                 if (b >= 0) {
                     int axis, spatial;
                     float split;
-                    split_decide(&S.box[0][b], kFinishSlots, by_position, axis, split, spatial);
-                    const int e = S.send[cur][b];
+                    split_decide(&S.box[0][b >> 1], kFinishSlots / 2, by_position, axis, split, spatial);
+                    const int e = S.send[cur][b >> 1];
                     f = spatial ? (S.c[axis][S.orig[cur][i]] < split ? 1 : 0)
                                 : ((i - b) < (e - b) / 2 ? 1 : 0);
                 }
@@ -1253,13 +1256,13 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
                 S.sid[cur ^ 1][i] = -1;  // no moving slot lands outside its own segment
                 continue;
             }
-            const int e = S.send[cur][b];
+            const int e = S.send[cur][b >> 1];
             const int fb = S.scan[b], mid = b + (S.scan[e] - fb), left_before = S.scan[i] - fb;
             const bool left = S.scan[i + 1] != S.scan[i];
             const int dest = left ? b + left_before : mid + ((i - b) - left_before);
             const int cb = left ? b : mid, ce = left ? mid : e;
             if (i == b) {
-                const int p = S.snode[cur][b];
+                const int p = S.snode[cur][b >> 1];
                 const int l = node_base + 2 * atomicAdd(&S.rank, 1), r = l + 1;  // r < cap
                 nfirst[l] = gb + b;
                 nlast[l] = gb + mid - 1;
@@ -1275,12 +1278,12 @@ __global__ void __launch_bounds__(kFinishThreads) k_split_finish(
                 for (int c = 0; c < 2; ++c) {
                     const int xb = c == 0 ? b : mid, xe = c == 0 ? mid : e;
                     if (xe - xb > K) {
-                        S.send[cur ^ 1][xb] = (short)xe;
-                        S.snode[cur ^ 1][xb] = l + c;
+                        S.send[cur ^ 1][xb >> 1] = (short)xe;
+                        S.snode[cur ^ 1][xb >> 1] = l + c;
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
-                            S.box[a][xb] = 0xffffffffu;
-                            S.box[3 + a][xb] = 0u;
+                            S.box[a][xb >> 1] = 0xffffffffu;
+                            S.box[3 + a][xb >> 1] = 0u;
                         }
                         atomicAdd(&S.ns[cur ^ 1], 1);
                     }
