@@ -12,7 +12,7 @@
 //       and rank(v) = #ancestors sharing first(v)
 //   K4  bottom-up FP64 refit of order-0/1/2 moments: leaves grouped by triangle count, one
 //       thread each; parents by recentring children, level by level over dense lists (split
-//       tree: its levels; LBVH: node heights from an integer atomic-counter ascent)
+//       tree as its levels are made, LBVH by its way up to the root)
 //   K4a exact node radii (farthest vertex, float screen + FP64 terms for the candidates), then
 //       conversion to 128 B FP32 / 256 B FP64 records in DFS order
 // The alternative top-down builders (FWN_BUILDER_SPLIT, FWN_BUILDER_BINNED) replace K1-K3b with
@@ -417,7 +417,7 @@ struct BuildState {
     int leaf_size[kLeafSizes]; // listed leaves by triangle count
     int leaf_next[kLeafSizes]; // of those, the ones k_leaf_sort has placed
     int2 level[kMaxLevels + 1];  // active segments; nodes made before
-    int internal[kMaxHeight];  // internal nodes by depth (split) or height (LBVH)
+    int internal[kMaxHeight];  // internal nodes by depth
 };
 struct LevelBound {
     int level, cap, segments;  // at most: nodes in all, active segments of a level
@@ -1639,6 +1639,179 @@ __global__ void k_refit(int num_leaves, const int* __restrict__ leaf_list,
     store_rec(&stage[pos[e]], R);
 }
 
+// The leaf pass of a build whose leaves do not fill the GPU (kLaneLeaves): G lanes per leaf, one
+// triangle each, then the leaf's 34 sums, one lane each over its triangles in order, then the
+// recentring, one result per lane. Every operation is leaf_moments's, with the same bits (an
+// addition as a fused multiply-add by one). What it saves is the chain of one thread's triangles;
+// where FP64 issue counts, the thread form's warps are fuller (leaves sorted by size).
+template <int G>
+__global__ void __launch_bounds__(32) k_refit_lanes(
+    int num_leaves, const int* __restrict__ leaf_list, const uint64_t* __restrict__ keys,
+    const int* __restrict__ first, const int* __restrict__ last, const int* __restrict__ pos,
+    const uint32_t* __restrict__ tri_of_slot, const float* __restrict__ V,
+    const int32_t* __restrict__ F, const int64_t* __restrict__ voff, StageRec* __restrict__ stage) {
+    constexpr int kLeaves = 32 / G, kSums = 34;
+    // a triangle's values: area, c[3], n[3], d[3], Q[6], one
+    constexpr int kArea = 0, kC = 1, kN = 4, kD = 7, kQ = 10, kOne = 16, kValues = 17;
+    __shared__ double val[kValues][32];
+    __shared__ double rec[kLeaves][kSums];  // sums: area, S[3], N[3], M1[9], M2[18]
+    __shared__ double ctr[kLeaves][6];      // P[3], e[3]
+    const int lane = threadIdx.x, g = lane / G, sub = lane % G;
+    const int k = blockIdx.x * kLeaves + g;
+    const bool on = k < num_leaves;
+    const int u = on ? leaf_list[k] : 0;
+    const int f = on ? first[u] : 0, cnt = on ? last[u] - f + 1 : 0;
+    const bool tri = sub < cnt;
+    float vf[3][3] = {};
+    double v[3][3] = {}, c[3], c0[3];
+    if (tri) {
+        const int64_t t = tri_of_slot[f + sub], base = voff[(int)(keys[f + sub] >> MORTON_BITS)];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const float* p = V + 3 * (base + F[3 * t + j]);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                vf[j][a] = p[a];
+                v[j][a] = f2d(vf[j][a]);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        c[a] = ((v[0][a] + v[1][a]) + v[2][a]) * kThird;
+        c0[a] = __shfl_sync(0xffffffffu, c[a], g * G);
+    }
+    const int SJ[6] = {0, 1, 2, 0, 0, 1};
+    const int SK[6] = {0, 1, 2, 1, 2, 2};
+    {
+        double e1[3], e2[3], nn[3], d[3], w[3][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            e1[a] = v[1][a] - v[0][a];
+            e2[a] = v[2][a] - v[0][a];
+        }
+        nn[0] = 0.5 * fmad(e1[1], e2[2], -(e1[2] * e2[1]));
+        nn[1] = 0.5 * fmad(e1[2], e2[0], -(e1[0] * e2[2]));
+        nn[2] = 0.5 * fmad(e1[0], e2[1], -(e1[1] * e2[0]));
+        val[kArea][lane] = sqrt(fmad(nn[0], nn[0], fmad(nn[1], nn[1], nn[2] * nn[2])));
+        val[kOne][lane] = 1.0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            d[a] = c[a] - c0[a];
+            val[kC + a][lane] = c[a];
+            val[kN + a][lane] = nn[a];
+            val[kD + a][lane] = d[a];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) w[j][a] = v[j][a] - c[a];
+        }
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int j = SJ[q], m = SK[q];
+            const double cov = fmad(w[0][j], w[0][m], fmad(w[1][j], w[1][m], w[2][j] * w[2][m])) * kTwelfth;
+            val[kQ + q][lane] = fmad(d[j], d[m], cov);
+        }
+    }
+    __syncwarp();
+    constexpr int kRounds = (kSums * kLeaves + 31) / 32;
+    double acc[kRounds];
+    int ix[kRounds], iy[kRounds], len[kRounds];
+    int most = 0;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int at = r * 32 + lane, leaf = min(at / kSums, kLeaves - 1), o = at % kSums;
+        const int x = o < 4 ? kArea : o < 7 ? kN + o - 4 : o < 16 ? kN + (o - 7) / 3 : kN + (o - 16) / 6;
+        const int y = o == 0 || (o >= 4 && o < 7) ? kOne : o < 4 ? kC + o - 1
+                      : o < 16 ? kD + (o - 7) % 3 : kQ + (o - 16) % 6;
+        ix[r] = x * 32 + leaf * G;
+        iy[r] = y * 32 + leaf * G;
+        acc[r] = 0.0;
+        const int n = __shfl_sync(0xffffffffu, cnt, leaf * G);
+        len[r] = at < kSums * kLeaves ? n : 0;
+        most = max(most, len[r]);
+    }
+    const double* flat = &val[0][0];
+    for (int t = 0; t < most; ++t)
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r)
+            if (t < len[r]) acc[r] = fmad(flat[ix[r] + t], flat[iy[r] + t], acc[r]);
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int at = r * 32 + lane;
+        if (at < kSums * kLeaves) rec[at / kSums][at % kSums] = acc[r];
+    }
+    __syncwarp();
+    // centre: the area-weighted mean, or for a leaf of zero area the plain mean of its centroids
+    const double A = rec[g][0];
+    if (sub < 3) {
+        double pe;
+        if (A > 0.0) {
+            pe = rec[g][1 + sub] / A;
+        } else {
+            double Cs = 0.0;
+            for (int t = 0; t < cnt; ++t) Cs = Cs + val[kC + sub][g * G + t];
+            pe = Cs / (double)cnt;
+        }
+        const double P = f2d(d2f(pe));
+        ctr[g][sub] = P;
+        ctr[g][3 + sub] = val[kC + sub][g * G] - P;
+    }
+    __syncwarp();
+    // radius: every vertex whose float estimate comes within 1e-5 of the largest (all of them near
+    // float's overflow), as in leaf_moments
+    const double P[3] = {ctr[g][0], ctr[g][1], ctr[g][2]};
+    const float Pf[3] = {d2f(P[0]), d2f(P[1]), d2f(P[2])};
+    float est[3], m = 0.f;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        est[j] = tri ? vertex_est(vf[j][0], vf[j][1], vf[j][2], Pf) : 0.f;
+        m = fmaxf(m, est[j]);
+    }
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float thr = m * 0.99999f - 1e-37f;
+    double r2 = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        if (tri && (!(m < INFINITY) || est[j] >= thr))
+            r2 = fmax(r2, vertex_r2(vf[j][0], vf[j][1], vf[j][2], P));
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+    // the records, about P
+    constexpr int kOut = 27 * kLeaves;
+#pragma unroll
+    for (int r = 0; r < (kOut + 31) / 32; ++r) {
+        const int at = r * 32 + lane, leaf = min(at / 27, kLeaves - 1), o = at % 27;
+        const int lu = __shfl_sync(0xffffffffu, u, leaf * G);
+        if (at >= kOut || blockIdx.x * kLeaves + leaf >= num_leaves) continue;
+        double* R = reinterpret_cast<double*>(stage + pos[lu]);
+        const double* N = &rec[leaf][4];
+        const double* M1 = &rec[leaf][7];
+        const double* e = &ctr[leaf][3];
+        if (o < 9) {
+            R[7 + o] = fmad(N[o / 3], e[o % 3], M1[o]);
+        } else {
+            const int i = (o - 9) / 6, q = (o - 9) % 6;
+            const int j = q < 3 ? q : q < 5 ? 0 : 1, n = q < 3 ? q : q == 3 ? 1 : 2;
+            R[16 + o - 9] = fmad(N[i], e[j] * e[n],
+                                 fmad(M1[3 * i + n], e[j], fmad(M1[3 * i + j], e[n], rec[leaf][16 + o - 9])));
+        }
+    }
+    if (on) {
+        double* R = reinterpret_cast<double*>(stage + pos[u]);
+        if (sub < 3) {
+            R[sub] = P[sub];
+            R[4 + sub] = rec[g][4 + sub];
+        }
+        if (sub == 3) R[3] = A;
+        if (sub == 4) R[34] = round_up_float(sqrt(r2));
+        if (sub == 5) R[35] = 0.0;
+    }
+}
+// 744 leaves of up to eight triangles take 14 us, 60 with a thread per leaf; 8,497 take 30 and 60,
+// 17,174 take 57 and 60. Of up to four, 7,200 take 23 and 33, 16,297 take 48 and 33; of up to
+// sixteen, 8,806 take 56 and 114.
+constexpr int kLaneLeaves = 12288;
+
 // The refit's leaf list grouped by triangle count (a counting sort over the sizes that the list's
 // maker counted), so that the 32 leaves of a warp run the same number of triangle iterations: the
 // FP64 pipe costs the same for a warp instruction whatever the number of active lanes.
@@ -1666,8 +1839,7 @@ __global__ void k_leaf_sort(int nl, const int* __restrict__ leaves, const int* _
     if (u >= 0) sorted[base[sz] + rank] = u;
 }
 
-// The internal nodes of one level of a split tree, or of one height of the LBVH
-// (nodes[0 .. count)): each combines its two children, whose records the leaf pass or an
+// The internal nodes of one depth (nodes[0 .. count)): each combines its two children, whose records the leaf pass or an
 // earlier (deeper, or lower) list wrote. A combine is some 270 FP64 instructions, and an SM issues
 // one FP64 warp instruction in 16 cycles, so the few warps of a small level are spread: one warp
 // per block (four to a block cost 10 us in the smallest levels), and levels that do not fill the
@@ -1705,11 +1877,12 @@ __global__ void __launch_bounds__(32) k_refit_level(int count, const int* __rest
 
 // The same combine (every operation of combine_moments, with the same bits) by four lanes: lane
 // i < 3 takes the i-th component of P and N and the i-th rows of M1 and M2.
-__global__ void __launch_bounds__(32) k_refit_level_lanes(
-    int count, const int* __restrict__ nodes, const int* __restrict__ left,
-    const int* __restrict__ right, const int* __restrict__ pos, StageRec* __restrict__ stage,
-    unsigned* __restrict__ status) {
-    const int k = (blockIdx.x * 32 + threadIdx.x) >> 2, i = threadIdx.x & 3;
+__device__ __forceinline__ void refit_lanes(int k, int count, const int* __restrict__ nodes,
+                                            const int* __restrict__ left,
+                                            const int* __restrict__ right,
+                                            const int* __restrict__ pos, StageRec* stage,
+                                            unsigned* __restrict__ status) {
+    const int i = threadIdx.x & 3;
     int p = -1, l = -1, r = -1;
     if (k < count && i < 3) {
         p = nodes[k];
@@ -1769,44 +1942,37 @@ __global__ void __launch_bounds__(32) k_refit_level_lanes(
         R[35] = 0.0;  // pad
     }
 }
+__global__ void __launch_bounds__(32) k_refit_level_lanes(
+    int count, const int* __restrict__ nodes, const int* __restrict__ left,
+    const int* __restrict__ right, const int* __restrict__ pos, StageRec* stage,
+    unsigned* __restrict__ status) {
+    refit_lanes((blockIdx.x * 32 + threadIdx.x) >> 2, count, nodes, left, right, pos, stage, status);
+}
+
+// The last levels, of at most kTopNodes nodes each, by one block: 3 us a level in place of a launch
+// each, 7 to 8 us.
+constexpr int kTopNodes = 32;
+constexpr int kTopLevels = 24;
+struct TopLevels {
+    int count[kTopLevels], start[kTopLevels];  // in the order that they are combined
+};
+__global__ void __launch_bounds__(4 * kTopNodes) k_refit_top(
+    int levels, TopLevels top, const int* __restrict__ order, const int* __restrict__ left,
+    const int* __restrict__ right, const int* __restrict__ pos, StageRec* stage,
+    unsigned* __restrict__ status) {
+    for (int l = 0; l < levels; ++l) {
+        refit_lanes(threadIdx.x >> 2, top.count[l], order + top.start[l], left, right, pos, stage,
+                    status);
+        __syncthreads();  // the next level reads what this one wrote
+    }
+}
 // At 8,192 nodes the two forms meet: the lane form takes 8 us there; the thread form 13 us at 16,000,
 // where the lane form's repeated address work and its 1.4 times as many FP64 instructions show.
 constexpr int kLaneLevel = 8192;
 
-// LBVH: the height of every emitted internal node (a leaf is 0, a node one more than its taller
-// child), by an integer ascent from the emitted leaves (the second child to arrive continues);
-// the FP64 combine then runs height by height over dense lists (k_refit_level), like the split
-// tree's levels, instead of on the ascent's ever sparser warps.
-__global__ void k_heights(const int* __restrict__ num_leaves, const int* __restrict__ leaf_list,
-                          const uint64_t* __restrict__ keys, const int* __restrict__ parent,
-                          const int* __restrict__ first, const int* __restrict__ last,
-                          int* __restrict__ visit, int* __restrict__ height,
-                          unsigned* __restrict__ status) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= *num_leaves) return;
-    int v = leaf_list[k], h = 0;
-    for (int guard = 0; v != 0; ++guard) {
-        const int p = parent[v];
-        if (p < 0) {  // in the LBVH only node 0 has no parent
-            atomicOr(status, ST_REFIT_ORPHAN);
-            return;
-        }
-        if (is_cross(keys, first, last, p)) return;  // v is a mesh root
-        if (guard >= kMaxHeight - 1) {
-            atomicOr(status, ST_REFIT_ORPHAN);
-            return;
-        }
-        atomicMax(&height[p], h + 1);
-        __threadfence();
-        if (atomicAdd(&visit[p], 1) == 0) return;  // first arrival: the sibling continues
-        __threadfence();
-        h = atomicAdd(&height[p], 0);  // both children's contributions are in
-        v = p;
-    }
-}
-
-// Counting sort of the emitted internal nodes (not spanning meshes) by height: hist[h] counts,
-// then (after an exclusive scan) list[offset[h] + rank] = node.
+// Counting sort of the emitted internal nodes (not spanning meshes) by depth: hist[d] counts, then
+// (after an exclusive scan) list[offset[d] + rank] = node. The split builders record the depths and
+// counts as they make the nodes.
 __device__ __forceinline__ bool refit_internal(const uint64_t* __restrict__ keys,
                                                const int* __restrict__ first,
                                                const int* __restrict__ last,
@@ -1815,26 +1981,36 @@ __device__ __forceinline__ bool refit_internal(const uint64_t* __restrict__ keys
     return (fl & 1) && !(fl & 2) && !is_cross(keys, first, last, u);
 }
 
-__global__ void k_height_hist(int nint, const uint64_t* __restrict__ keys,
-                              const int* __restrict__ first, const int* __restrict__ last,
-                              const uint8_t* __restrict__ flags, const int* __restrict__ height,
-                              int* __restrict__ hist, unsigned* __restrict__ status) {
+// LBVH: the depth of every emitted internal node, by its way up to the root (node 0), and the counts.
+__global__ void k_depths(int nint, const uint64_t* __restrict__ keys, const int* __restrict__ parent,
+                         const int* __restrict__ first, const int* __restrict__ last,
+                         const uint8_t* __restrict__ flags, int* __restrict__ depth,
+                         int* __restrict__ hist, unsigned* __restrict__ status) {
     __shared__ int h_s[kMaxHeight];  // the block's counts, then one atomic per non-zero entry
     for (int i = threadIdx.x; i < kMaxHeight; i += blockDim.x) h_s[i] = 0;
     __syncthreads();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u < nint && refit_internal(keys, first, last, flags, u)) {
-        if (height[u] < 0 || height[u] >= kMaxHeight) atomicOr(status, ST_REFIT_ORPHAN);
-        atomicAdd(&h_s[min(max(height[u], 0), kMaxHeight - 1)], 1);
+        int d = 0;
+        for (int v = u; v != 0 && d < kMaxHeight - 1; ++d) {
+            v = parent[v];
+            if (v < 0) {  // only node 0 has no parent
+                atomicOr(status, ST_REFIT_ORPHAN);
+                break;
+            }
+        }
+        if (d == kMaxHeight - 1) atomicOr(status, ST_REFIT_ORPHAN);
+        depth[u] = d;
+        atomicAdd(&h_s[d], 1);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kMaxHeight; i += blockDim.x)
         if (h_s[i]) atomicAdd(&hist[i], h_s[i]);
 }
 
-__global__ void k_height_sort(int nint, const uint64_t* __restrict__ keys,
+__global__ void k_depth_sort(int nint, const uint64_t* __restrict__ keys,
                               const int* __restrict__ first, const int* __restrict__ last,
-                              const uint8_t* __restrict__ flags, const int* __restrict__ height,
+                              const uint8_t* __restrict__ flags, const int* __restrict__ depth,
                               int* __restrict__ offset, int* __restrict__ list) {
     __shared__ int cnt[kMaxHeight];   // the block's nodes per key (ranks from shared atomics)
     __shared__ int base[kMaxHeight];  // where they go: one global atomic per non-zero key
@@ -1843,7 +2019,7 @@ __global__ void k_height_sort(int nint, const uint64_t* __restrict__ keys,
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     int h = -1, rank = 0;
     if (u < nint && refit_internal(keys, first, last, flags, u)) {
-        h = min(max(height[u], 0), kMaxHeight - 1);
+        h = min(max(depth[u], 0), kMaxHeight - 1);
         rank = atomicAdd(&cnt[h], 1);
     }
     __syncthreads();
@@ -2475,15 +2651,13 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         int* pos = arena.take<int>(cap);
         int* skip = arena.take<int>(cap);
         void* scan_tmp = arena.take<char>(exclusive_scan_temp_bytes(cap + 1));
-        int* visit = split ? nullptr : arena.take<int>(nint);
         int* leaf_list = arena.take<int>(n);
         int* leaf_list_len = &bst->leaf_list;
         const uint64_t* keys = nullptr;
         const uint32_t* tri_of_slot = nullptr;
         int num_nodes = 0;
-        std::vector<int> h_hist(kMaxHeight);  // internal nodes by depth or height
-        // split tree: every node's depth (roots 0), the order of the level-by-level refit
-        int* depth_of = split ? arena.take<int>(cap) : nullptr;
+        std::vector<int> h_hist(kMaxHeight);  // internal nodes by depth
+        int* depth_of = arena.take<int>(split ? cap : nint);  // (split tree: roots 0)
         auto check_input = [](unsigned st_h) {
             if (st_h & ST_BAD_INDEX) throw Error(FWN_INVALID_ARG, "triangle vertex index out of range");
             if (st_h & ST_NONFINITE)
@@ -2706,22 +2880,15 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             FWN_CUDA_CHECK(cudaGetLastError());
         }
         // internal nodes are refitted level by level, one thread per node of a dense list (an atomic
-        // ascent would leave most lanes of its warps idle on GB300's narrow FP64 pipe): the split
-        // tree deepest first by node depth, the LBVH lowest first by node height (k_heights)
-        int* key = depth_of;
+        // ascent would leave most lanes of its warps idle on GB300's narrow FP64 pipe), the deepest
+        // first
         int E = num_nodes, NL = 0;
         if (split) {  // every node is emitted, and all but the internal ones are leaves
             NL = num_nodes - std::accumulate(h_hist.begin(), h_hist.end(), 0);
         } else {
-            key = arena.take<int>(nint);
-            if (n > 1) {
-                FWN_CUDA_CHECK(cudaMemsetAsync(visit, 0, (size_t)nint * sizeof(int), st));
-                FWN_CUDA_CHECK(cudaMemsetAsync(key, 0, (size_t)nint * sizeof(int), st));
-                k_heights<<<grid_for(n, 128), 128, 0, st>>>(leaf_list_len, leaf_list, keys, parent,
-                                                            first, last, visit, key, status);
-                k_height_hist<<<grid_for(nint, 1024), 1024, 0, st>>>(nint, keys, first, last, flags, key,
-                                                                    bst->internal, status);
-            }
+            if (n > 1)
+                k_depths<<<grid_for(nint, 256), 256, 0, st>>>(nint, keys, parent, first, last, flags, depth_of,
+                                                             bst->internal, status);
             FWN_CUDA_CHECK(cudaMemcpyAsync(&bst->emitted, cnt + n, sizeof(int),
                                            cudaMemcpyDeviceToDevice, st));
             FWN_CUDA_CHECK(cudaGetLastError());
@@ -2742,17 +2909,19 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         // and a build that got less stops here rather than launch misaligned vector loads
         if (reinterpret_cast<uintptr_t>(stage) % alignof(StageRec) != 0)
             throw Error(FWN_INTERNAL, "staging records are not 32 B aligned");
-        if (NL > 0) {
+        if (NL > kLaneLeaves) {
             int* leaf_sorted = arena.take<int>(NL);
             k_leaf_sort<<<grid_for(NL, 256), 256, 0, st>>>(NL, leaf_list, first, last, bst,
                                                           leaf_sorted);
-            leaf_list = leaf_sorted;
-        }
-        if (NL > 0)
-            k_refit<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_list, keys, first, last, pos,
+            k_refit<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_sorted, keys, first, last, pos,
                                                        tri_of_slot, d_V, d_F, voff, stage);
+        } else if (NL > 0) {
+            const int per = K <= 8 ? 4 : 2;
+            (K <= 8 ? k_refit_lanes<8> : k_refit_lanes<16>)<<<grid_for(NL, per), 32, 0, st>>>(
+                NL, leaf_list, keys, first, last, pos, tri_of_slot, d_V, d_F, voff, stage);
+        }
         if (NL > 0 && n > 1) {
-            // the levels' lists come from one counting sort by depth or height
+            // the levels' lists come from one counting sort by depth
             const int count = split ? num_nodes : nint;
             int* offsets = arena.take<int>(kMaxHeight);
             int* order = arena.take<int>(count);
@@ -2760,10 +2929,12 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             for (int h = 0; h < kMaxHeight; ++h) off[h + 1] = off[h] + h_hist[h];
             FWN_CUDA_CHECK(cudaMemcpyAsync(offsets, off.data(), kMaxHeight * sizeof(int),
                                            cudaMemcpyHostToDevice, st));
-            k_height_sort<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, key,
+            k_depth_sort<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, depth_of,
                                                                 offsets, order);
-            for (int t = 0; t < kMaxHeight; ++t) {
-                const int h = split ? kMaxHeight - 1 - t : t;
+            TopLevels top{};
+            int tops = 0, h = kMaxHeight - 1;
+            while (tops < kTopLevels && h_hist[tops] <= kTopNodes && tops < kMaxHeight) ++tops;
+            for (; h >= tops; --h) {
                 if (h_hist[h] == 0) continue;
                 if (h_hist[h] <= kLaneLevel)
                     k_refit_level_lanes<<<grid_for(h_hist[h], 8), 32, 0, st>>>(
@@ -2772,6 +2943,15 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                     k_refit_level<<<grid_for(h_hist[h], 32), 32, 0, st>>>(
                         h_hist[h], order + off[h], left, right, pos, stage, status);
             }
+            int levels = 0;
+            for (; h >= 0; --h)
+                if (h_hist[h]) {
+                    top.count[levels] = h_hist[h];
+                    top.start[levels++] = off[h];
+                }
+            if (levels)
+                k_refit_top<<<1, 4 * kTopNodes, 0, st>>>(levels, top, order, left, right, pos, stage,
+                                                         status);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
         e.tris = static_cast<TriF32*>(engine_alloc((size_t)n * sizeof(TriF32), st));

