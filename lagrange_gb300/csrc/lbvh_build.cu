@@ -1360,6 +1360,26 @@ __device__ __forceinline__ float d2f(double x) {
     return __uint_as_float((hi & 0x80000000u) + (((e - 896u) << 23) | f) + up);
 }
 
+// x / 2 by the exponent, for the same reason.
+__device__ __forceinline__ double half_of(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+    if (((hi & 0x7fffffff) | lo) == 0) return x;  // +-0
+    if (e < 2u || e == 0x7ffu) return 0.5 * x;
+    return __hiloint2double(hi - 0x100000, lo);
+}
+
+// (float)(a / b) with one division for several a: from inv = 1 / b the quotient comes within two units
+// of the double a / b, which rounds to the same float unless it lies that close to the middle of
+// two floats; there (and outside float's normal range) the division itself decides.
+__device__ __forceinline__ float quotient_float(double a, double b, double inv) {
+    const double q = a * inv;
+    const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+    const int off = (__double2loint(q) & 0x1fffffff) - 0x10000000;
+    if (e < 897u || e > 1150u || (off >= -4 && off <= 4)) return d2f(a / b);
+    return d2f(q);
+}
+
 __device__ __forceinline__ double round_up_float(double x) {
     float f = d2f(x);
     if (f2d(f) < x) f = nextafterf(f, INFINITY);
@@ -1463,9 +1483,9 @@ __device__ void leaf_moments(const float* __restrict__ V, const int32_t* __restr
             e1[a] = v[1][a] - v[0][a];
             e2[a] = v[2][a] - v[0][a];
         }
-        nn[0] = 0.5 * fmad(e1[1], e2[2], -(e1[2] * e2[1]));
-        nn[1] = 0.5 * fmad(e1[2], e2[0], -(e1[0] * e2[2]));
-        nn[2] = 0.5 * fmad(e1[0], e2[1], -(e1[1] * e2[0]));
+        nn[0] = half_of(fmad(e1[1], e2[2], -(e1[2] * e2[1])));
+        nn[1] = half_of(fmad(e1[2], e2[0], -(e1[0] * e2[2])));
+        nn[2] = half_of(fmad(e1[0], e2[1], -(e1[1] * e2[0])));
         const double a_t = sqrt(fmad(nn[0], nn[0], fmad(nn[1], nn[1], nn[2] * nn[2])));
         for (int a = 0; a < 3; ++a) c[a] = ((v[0][a] + v[1][a]) + v[2][a]) * kThird;
         if (s == f)
@@ -1499,11 +1519,10 @@ __device__ void leaf_moments(const float* __restrict__ V, const int32_t* __restr
             load_tri_d(V, F, voff[(int)(keys[s] >> MORTON_BITS)], tri_of_slot[s], v);
             for (int a = 0; a < 3; ++a) Cs[a] = Cs[a] + ((v[0][a] + v[1][a]) + v[2][a]) * kThird;
         }
-    const double cnt = (double)(l - f + 1);
+    const double cnt = (double)(l - f + 1), over = A > 0.0 ? A : cnt, inv = 1.0 / over;
     double P[3], e[3];
     for (int a = 0; a < 3; ++a) {
-        const double pe = A > 0.0 ? S[a] / A : Cs[a] / cnt;
-        P[a] = f2d(d2f(pe));
+        P[a] = f2d(quotient_float(A > 0.0 ? S[a] : Cs[a], over, inv));
         e[a] = c0[a] - P[a];
     }
     for (int i = 0; i < 3; ++i) {
@@ -1583,11 +1602,11 @@ __device__ void combine_moments(const StageRec* __restrict__ a_, const StageRec*
     const double* Nb = hb + 4;
     const double* M1a = ha + 7;
     const double* M1b = hb + 7;
-    const double A = Aa + Ab;
+    const double A = Aa + Ab, inv = 1.0 / A;
     double P[3], ea[3], eb[3];
     for (int i = 0; i < 3; ++i) {
-        const double pe = A > 0.0 ? fmad(Aa, Pa[i], Ab * Pb[i]) / A : (Pa[i] + Pb[i]) * 0.5;
-        P[i] = f2d(d2f(pe));
+        P[i] = f2d(A > 0.0 ? quotient_float(fmad(Aa, Pa[i], Ab * Pb[i]), A, inv)
+                           : d2f((Pa[i] + Pb[i]) * 0.5));
         ea[i] = Pa[i] - P[i];
         eb[i] = Pb[i] - P[i];
     }
@@ -1690,9 +1709,9 @@ __global__ void __launch_bounds__(32) k_refit_lanes(
             e1[a] = v[1][a] - v[0][a];
             e2[a] = v[2][a] - v[0][a];
         }
-        nn[0] = 0.5 * fmad(e1[1], e2[2], -(e1[2] * e2[1]));
-        nn[1] = 0.5 * fmad(e1[2], e2[0], -(e1[0] * e2[2]));
-        nn[2] = 0.5 * fmad(e1[0], e2[1], -(e1[1] * e2[0]));
+        nn[0] = half_of(fmad(e1[1], e2[2], -(e1[2] * e2[1])));
+        nn[1] = half_of(fmad(e1[2], e2[0], -(e1[0] * e2[2])));
+        nn[2] = half_of(fmad(e1[0], e2[1], -(e1[1] * e2[0])));
         val[kArea][lane] = sqrt(fmad(nn[0], nn[0], fmad(nn[1], nn[1], nn[2] * nn[2])));
         val[kOne][lane] = 1.0;
 #pragma unroll
@@ -2331,19 +2350,20 @@ __device__ void derive_coeffs(const StageRec& R, Coeffs& c) {
     for (int k = 0; k < 3; ++k) {
         const double u = (m2(0, 0, k) + m2(1, 1, k)) + m2(2, 2, k);
         const double v = (m2(k, 0, 0) + m2(k, 1, 1)) + m2(k, 2, 2);
-        c.W[k] = -1.5 * (2.0 * u + v);
+        c.W[k] = -1.5 * fmad(2.0, u, v);  // (2 u is exact: one rounding either way)
     }
     // D = 7.5 * coefficients of the cubic sum_ijk M2_ijk d_i d_j d_k per monomial
     const double xxx = m2(0, 0, 0), yyy = m2(1, 1, 1), zzz = m2(2, 2, 2);
-    const double xxy = 2.0 * m2(0, 0, 1) + m2(1, 0, 0);
-    const double xxz = 2.0 * m2(0, 0, 2) + m2(2, 0, 0);
-    const double xyy = 2.0 * m2(1, 0, 1) + m2(0, 1, 1);
-    const double yyz = 2.0 * m2(1, 1, 2) + m2(2, 1, 1);
-    const double xzz = 2.0 * m2(2, 0, 2) + m2(0, 2, 2);
-    const double yzz = 2.0 * m2(2, 1, 2) + m2(1, 2, 2);
-    const double xyz = 2.0 * ((m2(0, 1, 2) + m2(1, 0, 2)) + m2(2, 0, 1));
-    const double mono[10] = {xxx, yyy, zzz, xxy, xxz, xyy, yyz, xzz, yzz, xyz};
-    for (int i = 0; i < 10; ++i) c.D[i] = 7.5 * mono[i];
+    const double xxy = fmad(2.0, m2(0, 0, 1), m2(1, 0, 0));
+    const double xxz = fmad(2.0, m2(0, 0, 2), m2(2, 0, 0));
+    const double xyy = fmad(2.0, m2(1, 0, 1), m2(0, 1, 1));
+    const double yyz = fmad(2.0, m2(1, 1, 2), m2(2, 1, 1));
+    const double xzz = fmad(2.0, m2(2, 0, 2), m2(0, 2, 2));
+    const double yzz = fmad(2.0, m2(2, 1, 2), m2(1, 2, 2));
+    const double xyz = (m2(0, 1, 2) + m2(1, 0, 2)) + m2(2, 0, 1);  // the half of its coefficient
+    const double mono[9] = {xxx, yyy, zzz, xxy, xxz, xyy, yyz, xzz, yzz};
+    for (int i = 0; i < 9; ++i) c.D[i] = 7.5 * mono[i];
+    c.D[9] = 15.0 * xyz;
 }
 
 // The emitted node at each DFS position (node_of_pos[pos[u]] = u), so that the conversion runs
