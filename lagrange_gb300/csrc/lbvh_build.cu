@@ -81,6 +81,7 @@ __device__ __forceinline__ int find_mesh(const int64_t* off, int nmeshes, int64_
 // ---- K0: per-mesh vertex bbox -----------------------------------------------------------------
 __global__ void k_mesh_bbox(const float* __restrict__ V, const int64_t* __restrict__ voff,
                             int chunk, unsigned* __restrict__ enc) {
+    after_previous();
     const int m = blockIdx.y;
     const int64_t v0 = voff[m] + (int64_t)blockIdx.x * chunk;
     const int64_t v1 = min(voff[m + 1], v0 + chunk);
@@ -112,6 +113,7 @@ __global__ void k_mesh_bbox(const float* __restrict__ V, const int64_t* __restri
 }
 
 __global__ void k_init_bbox(unsigned* enc, int nmeshes) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 6 * nmeshes) enc[i] = (i % 6) < 3 ? 0xffffffffu : 0u;
 }
@@ -119,6 +121,7 @@ __global__ void k_init_bbox(unsigned* enc, int nmeshes) {
 __global__ void k_mesh_info(const unsigned* __restrict__ enc, const int64_t* __restrict__ voff,
                             int nmeshes, float near_scale, float cond,
                             MeshInfo* __restrict__ mi) {
+    after_previous();
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nmeshes) return;
     MeshInfo r;
@@ -147,6 +150,7 @@ __global__ void k_tri_keys(const float* __restrict__ V, const int32_t* __restric
                            const int64_t* __restrict__ voff, const int64_t* __restrict__ foff,
                            int nmeshes, int64_t nf, const MeshInfo* __restrict__ mi,
                            uint64_t* __restrict__ keys, unsigned* __restrict__ status) {
+    after_previous();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nf) return;
     const int m = find_mesh(foff, nmeshes, t);
@@ -192,6 +196,7 @@ __device__ __forceinline__ int kdelta(const uint64_t* __restrict__ keys, int n, 
 }
 
 __global__ void k_leaf_init(int n, int* __restrict__ first, int* __restrict__ last) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     first[n - 1 + k] = k;
@@ -201,6 +206,7 @@ __global__ void k_leaf_init(int n, int* __restrict__ first, int* __restrict__ la
 __global__ void k_karras(const uint64_t* __restrict__ keys, int n, int* __restrict__ left,
                          int* __restrict__ right, int* __restrict__ parent,
                          int* __restrict__ first, int* __restrict__ last) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     const int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -301,6 +307,7 @@ __global__ void k_emit_count(int n, int K, const uint64_t* __restrict__ keys,
                              const int* __restrict__ last, int* __restrict__ cnt_first,
                              uint8_t* __restrict__ flags, int* __restrict__ leaf_list,
                              int* __restrict__ leaf_list_len, int* __restrict__ by_size) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     bool pred = false;
     if (u < 2 * n - 1) {
@@ -322,6 +329,7 @@ __global__ void k_positions(int num_nodes, const int* __restrict__ parent,
                             const int* __restrict__ first, const int* __restrict__ last,
                             const uint8_t* __restrict__ flags, const int* __restrict__ base,
                             int* __restrict__ pos, int* __restrict__ skip) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= num_nodes) return;
     if (!(flags[u] & 1)) {
@@ -345,6 +353,7 @@ __global__ void k_mesh_roots(int nmeshes, const int64_t* __restrict__ foff, int 
                              const int* __restrict__ parent, const int* __restrict__ first,
                              const int* __restrict__ last, const int* __restrict__ pos,
                              const int* __restrict__ skip, MeshInfo* __restrict__ mi) {
+    after_previous();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nmeshes) return;
     const int64_t lo = foff[m], hi = foff[m + 1] - 1;
@@ -511,6 +520,7 @@ __device__ __forceinline__ void box_clear_level(unsigned* __restrict__ box, int 
 }
 
 __global__ void k_split_box_init(int nact, unsigned* __restrict__ box) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < nact) box_clear_level(box, i);
 }
@@ -523,6 +533,7 @@ __global__ void k_split_init(const float* __restrict__ V, const int32_t* __restr
                              SplitSlots out, int* __restrict__ final_perm,
                              uint64_t* __restrict__ keys, unsigned* __restrict__ box,
                              bool box_copies, unsigned* __restrict__ status) {
+    after_previous();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int key = -1;
     float c[3] = {0.f, 0.f, 0.f};
@@ -594,6 +605,7 @@ __global__ void k_split_decide(const BuildState* __restrict__ bst, LevelBound lb
                                const unsigned* __restrict__ box, int* __restrict__ axis_of,
                                float* __restrict__ split_of, int* __restrict__ spatial_of,
                                float* __restrict__ seg_box) {
+    after_previous();
     const int sg = blockIdx.x * blockDim.x + threadIdx.x;
     const int nact = level_segments(bst, lb);
     if (sg >= nact) return;
@@ -618,6 +630,7 @@ __global__ void k_split_decide(const BuildState* __restrict__ bst, LevelBound lb
 
 __global__ void k_split_bins_init(const BuildState* __restrict__ bst, LevelBound lb,
                                   unsigned* __restrict__ bins) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nwords = level_segments(bst, lb) * kSegBinWords;
     if (i >= nwords) return;
@@ -632,6 +645,7 @@ __global__ void __launch_bounds__(256) k_split_bins(int64_t n, BuildState* __res
                                                     LevelBound lb, SplitSlots cur,
                                                     const float* __restrict__ seg_box,
                                                     unsigned* __restrict__ bins) {
+    after_previous();
     if (level_segments(bst, lb) == 0) return;
     constexpr int kLocal = 4;
     __shared__ int tab[kLocal];
@@ -785,6 +799,7 @@ __global__ void k_split_choose(const BuildState* __restrict__ bst, LevelBound lb
                                const float* __restrict__ seg_box,
                                const unsigned* __restrict__ bins, int* __restrict__ axis_of,
                                int* __restrict__ bin_of, int* __restrict__ spatial_of) {
+    after_previous();
     const int sg = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (sg >= level_segments(bst, lb)) return;  // warp-uniform
@@ -879,6 +894,7 @@ k_split_flags(int64_t n, BuildState* __restrict__ bst, LevelBound lb, SplitSlots
               const unsigned* __restrict__ box, const int* __restrict__ axis_of,
               const float* __restrict__ split_of, const int* __restrict__ spatial_of,
               const int* __restrict__ bin_of, const float* __restrict__ seg_box, LeftRanks ranks) {
+    after_previous();
     constexpr int kRounds = kSplitTile / kFlagThreads, kWarps = kFlagThreads / 32;
     __shared__ struct { int seg, axis, spatial; float split; } sp[2];
     __shared__ int wc[kSplitTile / 32];
@@ -1019,6 +1035,7 @@ __global__ void k_split_children(BuildState* __restrict__ bst, LevelBound lb, in
                                  int* __restrict__ n_node, unsigned* __restrict__ n_box,
                                  int4* __restrict__ small, int4* __restrict__ part,
                                  int2* __restrict__ child_next) {
+    after_previous();
     const int sg = blockIdx.x * blockDim.x + threadIdx.x;
     const int nact = level_segments(bst, lb), node_base = bst->level[lb.level].y;
     if (sg == 0) {
@@ -1066,6 +1083,7 @@ __global__ void k_split_scatter(int64_t n, const BuildState* __restrict__ bst, L
                                 SplitSlots cur, SplitSlots nxt, LeftRanks ranks,
                                 const int4* __restrict__ part, const int2* __restrict__ child_next,
                                 int* __restrict__ final_perm, unsigned* __restrict__ n_box) {
+    after_previous();
     if (level_segments(bst, lb) == 0) return;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int key = -1;
@@ -1156,6 +1174,7 @@ __global__ void __launch_bounds__(kFinishThreads, 4) k_split_finish(
     int level_nodes, int cap, int* __restrict__ nfirst, int* __restrict__ nlast,
     int* __restrict__ nparent, int* __restrict__ nleft, int* __restrict__ nright,
     int* __restrict__ depth_of, int* __restrict__ final_perm) {
+    after_previous();
     unsigned* status = &bst->status;
     extern __shared__ __align__(16) unsigned char finish_smem[];
     FinishShared& S = *reinterpret_cast<FinishShared*>(finish_smem);
@@ -1310,6 +1329,7 @@ __global__ void k_split_emit(int num_nodes, const int* __restrict__ nfirst,
                              uint8_t* __restrict__ flags, int* __restrict__ cnt_first,
                              int* __restrict__ leaf_list, int* __restrict__ leaf_list_len,
                              int* __restrict__ by_size) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     bool leaf = false;
     if (u < num_nodes) {
@@ -1325,6 +1345,7 @@ __global__ void k_split_emit(int num_nodes, const int* __restrict__ nfirst,
 __global__ void k_split_mesh_roots(int nmeshes, const int* __restrict__ root_node,
                                    const int* __restrict__ pos, const int* __restrict__ skip,
                                    MeshInfo* __restrict__ mi) {
+    after_previous();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nmeshes) return;
     const int r = root_node[m];
@@ -1650,6 +1671,7 @@ __global__ void k_refit(int num_leaves, const int* __restrict__ leaf_list,
                         const uint32_t* __restrict__ tri_of_slot, const float* __restrict__ V,
                         const int32_t* __restrict__ F, const int64_t* __restrict__ voff,
                         StageRec* __restrict__ stage) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= num_leaves) return;
     const int e = leaf_list[k];
@@ -1669,6 +1691,7 @@ __global__ void __launch_bounds__(32) k_refit_lanes(
     const int* __restrict__ first, const int* __restrict__ last, const int* __restrict__ pos,
     const uint32_t* __restrict__ tri_of_slot, const float* __restrict__ V,
     const int32_t* __restrict__ F, const int64_t* __restrict__ voff, StageRec* __restrict__ stage) {
+    after_previous();
     constexpr int kLeaves = 32 / G, kSums = 34;
     // a triangle's values: area, c[3], n[3], d[3], Q[6], one
     constexpr int kArea = 0, kC = 1, kN = 4, kD = 7, kQ = 10, kOne = 16, kValues = 17;
@@ -1837,6 +1860,7 @@ constexpr int kLaneLeaves = 12288;
 __global__ void k_leaf_sort(int nl, const int* __restrict__ leaves, const int* __restrict__ first,
                             const int* __restrict__ last, BuildState* __restrict__ bst,
                             int* __restrict__ sorted) {
+    after_previous();
     __shared__ int cnt[kLeafSizes];   // the block's leaves per size (ranks from shared atomics)
     __shared__ int base[kLeafSizes];  // where they go: one global atomic per non-zero size
     if (threadIdx.x < kLeafSizes) cnt[threadIdx.x] = 0;
@@ -1884,6 +1908,7 @@ __global__ void __launch_bounds__(32) k_refit_level(int count, const int* __rest
                               const int* __restrict__ left, const int* __restrict__ right,
                               const int* __restrict__ pos, StageRec* __restrict__ stage,
                               unsigned* __restrict__ status) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int p = nodes[k];
@@ -1965,6 +1990,7 @@ __global__ void __launch_bounds__(32) k_refit_level_lanes(
     int count, const int* __restrict__ nodes, const int* __restrict__ left,
     const int* __restrict__ right, const int* __restrict__ pos, StageRec* stage,
     unsigned* __restrict__ status) {
+    after_previous();
     refit_lanes((blockIdx.x * 32 + threadIdx.x) >> 2, count, nodes, left, right, pos, stage, status);
 }
 
@@ -1979,6 +2005,7 @@ __global__ void __launch_bounds__(4 * kTopNodes) k_refit_top(
     int levels, TopLevels top, const int* __restrict__ order, const int* __restrict__ left,
     const int* __restrict__ right, const int* __restrict__ pos, StageRec* stage,
     unsigned* __restrict__ status) {
+    after_previous();
     for (int l = 0; l < levels; ++l) {
         refit_lanes(threadIdx.x >> 2, top.count[l], order + top.start[l], left, right, pos, stage,
                     status);
@@ -2005,6 +2032,7 @@ __global__ void k_depths(int nint, const uint64_t* __restrict__ keys, const int*
                          const int* __restrict__ first, const int* __restrict__ last,
                          const uint8_t* __restrict__ flags, int* __restrict__ depth,
                          int* __restrict__ hist, unsigned* __restrict__ status) {
+    after_previous();
     __shared__ int h_s[kMaxHeight];  // the block's counts, then one atomic per non-zero entry
     for (int i = threadIdx.x; i < kMaxHeight; i += blockDim.x) h_s[i] = 0;
     __syncthreads();
@@ -2031,6 +2059,7 @@ __global__ void k_depth_sort(int nint, const uint64_t* __restrict__ keys,
                               const int* __restrict__ first, const int* __restrict__ last,
                               const uint8_t* __restrict__ flags, const int* __restrict__ depth,
                               int* __restrict__ offset, int* __restrict__ list) {
+    after_previous();
     __shared__ int cnt[kMaxHeight];   // the block's nodes per key (ranks from shared atomics)
     __shared__ int base[kMaxHeight];  // where they go: one global atomic per non-zero key
     for (int i = threadIdx.x; i < kMaxHeight; i += blockDim.x) cnt[i] = 0;
@@ -2174,6 +2203,7 @@ __global__ void k_radius_list(int num_nodes, const uint64_t* __restrict__ keys,
                               const int* __restrict__ first, const int* __restrict__ last,
                               const uint8_t* __restrict__ flags, BuildState* __restrict__ bst,
                               int* __restrict__ list, int2* __restrict__ chunks, int max_chunks) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     const bool node = u < num_nodes && internal_emitted(keys, first, last, flags, u);
     const int f = node ? first[u] : 0, size = node ? last[u] - f + 1 : 0;
@@ -2230,6 +2260,7 @@ k_node_radius_listed(const int* __restrict__ list, int step, const int* __restri
                      const int* __restrict__ pos, const StageRec* __restrict__ stage,
                      const TriF32* __restrict__ tris, const float4* __restrict__ groups,
                      unsigned long long* __restrict__ r2bits) {
+    after_previous();
     static_assert(LANES == 8 || LANES == 32, "a node's lanes: eight or the warp");
     constexpr int kNodes = 32 / LANES;  // nodes a warp has in hand
     __shared__ RadiusQueue queues[kRadiusWarps];
@@ -2308,6 +2339,7 @@ __global__ void k_node_radius(const int2* __restrict__ chunks, const int* __rest
                               const int* __restrict__ pos, const StageRec* __restrict__ stage,
                               const TriF32* __restrict__ tris, const float4* __restrict__ groups,
                               unsigned long long* __restrict__ r2bits) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int total = min(*count, max_chunks);
     const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
@@ -2371,6 +2403,7 @@ __device__ void derive_coeffs(const StageRec& R, Coeffs& c) {
 // and a thread per Karras node leaves the FP64 work of the conversion on sparse warps.
 __global__ void k_node_of_pos(int num_nodes, const uint8_t* __restrict__ flags,
                               const int* __restrict__ pos, int* __restrict__ node_of_pos) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u < num_nodes && (flags[u] & 1)) node_of_pos[pos[u]] = u;
 }
@@ -2382,6 +2415,7 @@ __global__ void k_convert(int num_records, const int* __restrict__ node_of_pos,
                           StageRec* __restrict__ stage, const unsigned long long* __restrict__ r2bits,
                           NodeF32* __restrict__ n32, NodeF64* __restrict__ n64,
                           int* __restrict__ leaf_count) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int u = i < num_records ? node_of_pos[i] : 0;
     const bool cross = i < num_records && is_cross(keys, first, last, u);
@@ -2443,6 +2477,7 @@ __global__ void k_convert(int num_records, const int* __restrict__ node_of_pos,
 // soa[k * num_nodes + i].
 __global__ void k_aos_to_soa(int64_t num_nodes, const NodeF32* __restrict__ n32,
                              float4* __restrict__ soa) {
+    after_previous();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_nodes) return;
     const float4* r = reinterpret_cast<const float4*>(n32 + i);
@@ -2455,6 +2490,7 @@ __global__ void k_tri_records(int n, const uint32_t* __restrict__ tri_of_slot,
                               const int32_t* __restrict__ F, const int64_t* __restrict__ voff,
                               TriF32* __restrict__ tris, int* __restrict__ sorted_tri,
                               float4* __restrict__ groups) {
+    after_previous();
     const int at = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = min(at, n - 1);  // (the lanes past the end stay for the group's reductions)
     const int64_t t = tri_of_slot[s];
@@ -2640,17 +2676,16 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
     StateReader reader(bst, st);
     unsigned* status = &bst->status;
     FWN_CUDA_CHECK(cudaMemsetAsync(bst, 0, sizeof(BuildState), st));
-    k_init_bbox<<<grid_for(6 * nmeshes, 256), 256, 0, st>>>(enc, (int)nmeshes);
+    launch_after(k_init_bbox, grid_for(6 * nmeshes, 256), 256, 0, st, enc, (int)nmeshes);
     int64_t maxv = 0;
     for (int64_t m = 0; m < nmeshes; ++m) maxv = std::max(maxv, voff_h[m + 1] - voff_h[m]);
     if (maxv > 0) {
         const int chunk = 16384;
         dim3 g((unsigned)((maxv + chunk - 1) / chunk), (unsigned)nmeshes);
-        k_mesh_bbox<<<g, 256, 0, st>>>(d_V, voff, chunk, enc);
+        launch_after(k_mesh_bbox, g, 256, 0, st, d_V, voff, chunk, enc);
     }
-    k_mesh_info<<<grid_for(nmeshes, 128), 128, 0, st>>>(enc, voff, (int)nmeshes,
-                                                        e.cfg.fp64_near_scale, e.cfg.fp64_cond,
-                                                        e.meshes);
+    launch_after(k_mesh_info, grid_for(nmeshes, 128), 128, 0, st, enc, voff, (int)nmeshes,
+        e.cfg.fp64_near_scale, e.cfg.fp64_cond, e.meshes);
     FWN_CUDA_CHECK(cudaGetLastError());
 
     if (nf > 0) {
@@ -2693,8 +2728,8 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             uint32_t* vals_b = arena.take<uint32_t>(n);
             void* sort_tmp = arena.take<char>(radix_sort_temp_bytes(n, 8));
             NvtxRange trace_keys("fwn build: Morton keys + sort");
-            k_tri_keys<<<grid_for(n, 256), 256, 0, st>>>(d_V, d_F, voff, foff, (int)nmeshes, nf,
-                                                         e.meshes, keys_a, status);
+            launch_after(k_tri_keys, grid_for(n, 256), 256, 0, st, d_V, d_F, voff, foff,
+                (int)nmeshes, nf, e.meshes, keys_a, status);
             FWN_CUDA_CHECK(cudaGetLastError());
             const bool in_b = radix_sort_u64(keys_a, vals_a, keys_b, vals_b, n,
                                              0, MORTON_BITS + mesh_bits, sort_tmp, st);
@@ -2705,21 +2740,22 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             num_nodes = nn;
             NvtxRange trace_tree("fwn build: Karras tree + DFS layout");
             FWN_CUDA_CHECK(cudaMemsetAsync(parent, 0xff, (size_t)nn * sizeof(int), st));  // -1
-            k_leaf_init<<<grid_for(n, 256), 256, 0, st>>>(n, first, last);
+            launch_after(k_leaf_init, grid_for(n, 256), 256, 0, st, n, first, last);
             if (n == 1) {
                 int m1 = -1;
                 FWN_CUDA_CHECK(cudaMemcpyAsync(parent, &m1, sizeof(int), cudaMemcpyHostToDevice, st));
             } else {
-                k_karras<<<grid_for(n - 1, 256), 256, 0, st>>>(keys, n, left, right, parent, first, last);
+                launch_after(k_karras, grid_for(n - 1, 256), 256, 0, st, keys, n, left, right,
+                    parent, first, last);
             }
             FWN_CUDA_CHECK(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(int), st));
-            k_emit_count<<<grid_for(nn, 256), 256, 0, st>>>(n, K, keys, parent, first, last, cnt, flags,
-                                                            leaf_list, leaf_list_len,
-                                                            bst->leaf_size);
+            launch_after(k_emit_count, grid_for(nn, 256), 256, 0, st, n, K, keys, parent, first,
+                last, cnt, flags, leaf_list, leaf_list_len, bst->leaf_size);
             exclusive_scan_i32(cnt, n + 1, scan_tmp, st);
-            k_positions<<<grid_for(nn, 256), 256, 0, st>>>(nn, parent, first, last, flags, cnt, pos, skip);
-            k_mesh_roots<<<grid_for(nmeshes, 128), 128, 0, st>>>((int)nmeshes, foff, n, parent, first,
-                                                                 last, pos, skip, e.meshes);
+            launch_after(k_positions, grid_for(nn, 256), 256, 0, st, nn, parent, first, last,
+                flags, cnt, pos, skip);
+            launch_after(k_mesh_roots, grid_for(nmeshes, 128), 128, 0, st, (int)nmeshes, foff, n,
+                parent, first, last, pos, skip, e.meshes);
         } else {
             NvtxRange trace_tree("fwn build: top-down splits + DFS layout");
             // roots: one node per non-empty mesh; a mesh of > kFinishSlots triangles is an active
@@ -2802,11 +2838,11 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                                cudaMemcpyHostToDevice, st));
                 FWN_CUDA_CHECK(cudaMemcpyAsync(seg_a[2], s_node.data(), nact * sizeof(int),
                                                cudaMemcpyHostToDevice, st));
-                k_split_box_init<<<grid_for(nact, 256), 256, 0, st>>>(nact, box_a);
+                launch_after(k_split_box_init, grid_for(nact, 256), 256, 0, st, nact, box_a);
             }
-            k_split_init<<<grid_for(n, 256), 256, 0, st>>>(d_V, d_F, voff, foff, (int)nmeshes, nf,
-                                                           d_mesh_seg, A, final_perm, skeys, box_a,
-                                                           nact <= kBoxCopyKeys, status);
+            launch_after(k_split_init, grid_for(n, 256), 256, 0, st, d_V, d_F, voff, foff,
+                (int)nmeshes, nf, d_mesh_seg, A, final_perm, skeys, box_a, nact <= kBoxCopyKeys,
+                status);
             FWN_CUDA_CHECK(cudaGetLastError());
             // A mesh of m triangles has segments to split for at least log2(m / kFinishSlots)
             // levels: the host launches those without looking. From there on level l + 1 is
@@ -2833,25 +2869,25 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                 const LevelBound lb{level, cap, seg_bound};
                 const int most = (int)std::min<int64_t>(seg_bound, (int64_t)nact << std::min(level, 30));
                 if (binned) {
-                    k_split_decide<<<grid_for(most, 128), 128, 0, st>>>(
-                        bst, lb, box_a, axis_of, split_of, spatial_of, seg_box);
+                    launch_after(k_split_decide, grid_for(most, 128), 128, 0, st, bst, lb, box_a,
+                        axis_of, split_of, spatial_of, seg_box);
                     if (level < kSpatialLevels) {  // the binned plane of each segment
-                        k_split_bins_init<<<grid_for((int64_t)most * kSegBinWords, 256), 256, 0, st>>>(
-                            bst, lb, bins);
-                        k_split_bins<<<(int)((n + kBinChunk - 1) / kBinChunk), 256, 0, st>>>(
-                            n, bst, lb, *cur, seg_box, bins);
-                        k_split_choose<<<grid_for(32 * (int64_t)most, 128), 128, 0, st>>>(
-                            bst, lb, seg_box, bins, axis_of, bin_of, spatial_of);
+                        launch_after(k_split_bins_init, grid_for((int64_t)most * kSegBinWords,
+                            256), 256, 0, st, bst, lb, bins);
+                        launch_after(k_split_bins, (int)((n + kBinChunk - 1) / kBinChunk), 256, 0,
+                            st, n, bst, lb, *cur, seg_box, bins);
+                        launch_after(k_split_choose, grid_for(32 * (int64_t)most, 128), 128, 0,
+                            st, bst, lb, seg_box, bins, axis_of, bin_of, spatial_of);
                     }
                 }
-                (binned ? k_split_flags<true> : k_split_flags<false>)<<<tiles, kFlagThreads, 0, st>>>(
-                    n, bst, lb, *cur, seg_a[0], seg_a[1], box_a, axis_of, split_of, spatial_of,
-                    bin_of, seg_box, ranks);
-                k_split_children<<<grid_for(most, 128), 128, 0, st>>>(
-                    bst, lb, K, seg_a[0], seg_a[1], seg_a[2], ranks, first, last, parent, left,
-                    right, depth_of, seg_b[0], seg_b[1], seg_b[2], box_b, small, part, child_next);
-                k_split_scatter<<<grid_for(n, 256), 256, 0, st>>>(n, bst, lb, *cur, *nxt, ranks, part,
-                                                                 child_next, final_perm, box_b);
+                launch_after(binned ? k_split_flags<true> : k_split_flags<false>, tiles,
+                    kFlagThreads, 0, st, n, bst, lb, *cur, seg_a[0], seg_a[1], box_a, axis_of,
+                    split_of, spatial_of, bin_of, seg_box, ranks);
+                launch_after(k_split_children, grid_for(most, 128), 128, 0, st, bst, lb, K,
+                    seg_a[0], seg_a[1], seg_a[2], ranks, first, last, parent, left, right,
+                    depth_of, seg_b[0], seg_b[1], seg_b[2], box_b, small, part, child_next);
+                launch_after(k_split_scatter, grid_for(n, 256), 256, 0, st, n, bst, lb, *cur,
+                    *nxt, ranks, part, child_next, final_perm, box_b);
                 FWN_CUDA_CHECK(cudaGetLastError());
                 if (level + 1 >= sure) reader.request(level & 1);
                 if (level >= sure) {
@@ -2874,9 +2910,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                 FWN_CUDA_CHECK(cudaFuncSetAttribute(k_split_finish,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)sizeof(FinishShared)));
-                k_split_finish<<<nsmall, kFinishThreads, sizeof(FinishShared), st>>>(
-                    small, A, B, K, bst, level_nodes, cap, first, last, parent, left, right, depth_of,
-                    final_perm);
+                launch_after(k_split_finish, nsmall, kFinishThreads, sizeof(FinishShared), st,
+                    small, A, B, K, bst, level_nodes, cap, first, last, parent, left, right,
+                    depth_of, final_perm);
                 FWN_CUDA_CHECK(cudaGetLastError());
             }
             reader.request(0);
@@ -2889,14 +2925,13 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             keys = skeys;
             tri_of_slot = reinterpret_cast<const uint32_t*>(final_perm);
             FWN_CUDA_CHECK(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(int), st));
-            k_split_emit<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, first, last, left,
-                                                                   flags, cnt, leaf_list,
-                                                                   leaf_list_len, bst->leaf_size);
+            launch_after(k_split_emit, grid_for(num_nodes, 256), 256, 0, st, num_nodes, first,
+                last, left, flags, cnt, leaf_list, leaf_list_len, bst->leaf_size);
             exclusive_scan_i32(cnt, n + 1, scan_tmp, st);
-            k_positions<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, parent, first, last,
-                                                                  flags, cnt, pos, skip);
-            k_split_mesh_roots<<<grid_for(nmeshes, 128), 128, 0, st>>>((int)nmeshes, d_root_node,
-                                                                       pos, skip, e.meshes);
+            launch_after(k_positions, grid_for(num_nodes, 256), 256, 0, st, num_nodes, parent,
+                first, last, flags, cnt, pos, skip);
+            launch_after(k_split_mesh_roots, grid_for(nmeshes, 128), 128, 0, st, (int)nmeshes,
+                d_root_node, pos, skip, e.meshes);
             FWN_CUDA_CHECK(cudaGetLastError());
         }
         // internal nodes are refitted level by level, one thread per node of a dense list (an atomic
@@ -2907,8 +2942,8 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             NL = num_nodes - std::accumulate(h_hist.begin(), h_hist.end(), 0);
         } else {
             if (n > 1)
-                k_depths<<<grid_for(nint, 256), 256, 0, st>>>(nint, keys, parent, first, last, flags, depth_of,
-                                                             bst->internal, status);
+                launch_after(k_depths, grid_for(nint, 256), 256, 0, st, nint, keys, parent, first,
+                    last, flags, depth_of, bst->internal, status);
             FWN_CUDA_CHECK(cudaMemcpyAsync(&bst->emitted, cnt + n, sizeof(int),
                                            cudaMemcpyDeviceToDevice, st));
             FWN_CUDA_CHECK(cudaGetLastError());
@@ -2931,14 +2966,14 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             throw Error(FWN_INTERNAL, "staging records are not 32 B aligned");
         if (NL > kLaneLeaves) {
             int* leaf_sorted = arena.take<int>(NL);
-            k_leaf_sort<<<grid_for(NL, 256), 256, 0, st>>>(NL, leaf_list, first, last, bst,
-                                                          leaf_sorted);
-            k_refit<<<grid_for(NL, 128), 128, 0, st>>>(NL, leaf_sorted, keys, first, last, pos,
-                                                       tri_of_slot, d_V, d_F, voff, stage);
+            launch_after(k_leaf_sort, grid_for(NL, 256), 256, 0, st, NL, leaf_list, first, last,
+                bst, leaf_sorted);
+            launch_after(k_refit, grid_for(NL, 128), 128, 0, st, NL, leaf_sorted, keys, first,
+                last, pos, tri_of_slot, d_V, d_F, voff, stage);
         } else if (NL > 0) {
             const int per = K <= 8 ? 4 : 2;
-            (K <= 8 ? k_refit_lanes<8> : k_refit_lanes<16>)<<<grid_for(NL, per), 32, 0, st>>>(
-                NL, leaf_list, keys, first, last, pos, tri_of_slot, d_V, d_F, voff, stage);
+            launch_after(K <= 8 ? k_refit_lanes<8> : k_refit_lanes<16>, grid_for(NL, per), 32, 0,
+                st, NL, leaf_list, keys, first, last, pos, tri_of_slot, d_V, d_F, voff, stage);
         }
         if (NL > 0 && n > 1) {
             // the levels' lists come from one counting sort by depth
@@ -2949,19 +2984,19 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             for (int h = 0; h < kMaxHeight; ++h) off[h + 1] = off[h] + h_hist[h];
             FWN_CUDA_CHECK(cudaMemcpyAsync(offsets, off.data(), kMaxHeight * sizeof(int),
                                            cudaMemcpyHostToDevice, st));
-            k_depth_sort<<<grid_for(count, 1024), 1024, 0, st>>>(count, keys, first, last, flags, depth_of,
-                                                                offsets, order);
+            launch_after(k_depth_sort, grid_for(count, 1024), 1024, 0, st, count, keys, first,
+                last, flags, depth_of, offsets, order);
             TopLevels top{};
             int tops = 0, h = kMaxHeight - 1;
             while (tops < kTopLevels && h_hist[tops] <= kTopNodes && tops < kMaxHeight) ++tops;
             for (; h >= tops; --h) {
                 if (h_hist[h] == 0) continue;
                 if (h_hist[h] <= kLaneLevel)
-                    k_refit_level_lanes<<<grid_for(h_hist[h], 8), 32, 0, st>>>(
+                    launch_after(k_refit_level_lanes, grid_for(h_hist[h], 8), 32, 0, st,
                         h_hist[h], order + off[h], left, right, pos, stage, status);
                 else
-                    k_refit_level<<<grid_for(h_hist[h], 32), 32, 0, st>>>(
-                        h_hist[h], order + off[h], left, right, pos, stage, status);
+                    launch_after(k_refit_level, grid_for(h_hist[h], 32), 32, 0, st, h_hist[h],
+                        order + off[h], left, right, pos, stage, status);
             }
             int levels = 0;
             for (; h >= 0; --h)
@@ -2970,15 +3005,15 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                     top.start[levels++] = off[h];
                 }
             if (levels)
-                k_refit_top<<<1, 4 * kTopNodes, 0, st>>>(levels, top, order, left, right, pos, stage,
-                                                         status);
+                launch_after(k_refit_top, 1, 4 * kTopNodes, 0, st, levels, top, order, left,
+                    right, pos, stage, status);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
         e.tris = static_cast<TriF32*>(engine_alloc((size_t)n * sizeof(TriF32), st));
         e.sorted_tri = static_cast<int*>(engine_alloc((size_t)n * sizeof(int), st));
         float4* groups = arena.take<float4>((n + kGroup - 1) / kGroup);
-        k_tri_records<<<grid_for(n, 256), 256, 0, st>>>(n, tri_of_slot, keys, d_V, d_F, voff,
-                                                        e.tris, e.sorted_tri, groups);
+        launch_after(k_tri_records, grid_for(n, 256), 256, 0, st, n, tri_of_slot, keys, d_V, d_F,
+            voff, e.tris, e.sorted_tri, groups);
         // exact radii of the internal nodes from the triangle records
         unsigned long long* r2bits = arena.take<unsigned long long>(E);
         FWN_CUDA_CHECK(cudaMemsetAsync(r2bits, 0, (size_t)E * sizeof(unsigned long long), st));
@@ -2990,19 +3025,18 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             // a level's larger nodes are n / kRadiusChunk at most, with as many whole chunks
             const int max_chunks = 2 * kMaxHeight * (n / kRadiusChunk);
             int2* chunks = arena.take<int2>(max_chunks);
-            k_radius_list<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, keys, first, last,
-                                                                    flags, bst, rlist, chunks,
-                                                                    max_chunks);
+            launch_after(k_radius_list, grid_for(num_nodes, 256), 256, 0, st, num_nodes, keys,
+                first, last, flags, bst, rlist, chunks, max_chunks);
             const int threads = 32 * kRadiusWarps;
-            k_node_radius_listed<8><<<sms * 8, threads, 0, st>>>(
-                rlist, 1, &bst->radius_tiny, first, last, pos, stage, e.tris, groups, r2bits);
+            launch_after(k_node_radius_listed<8>, sms * 8, threads, 0, st, rlist, 1,
+                &bst->radius_tiny, first, last, pos, stage, e.tris, groups, r2bits);
             if (n > kTinyNode)
-                k_node_radius_listed<32><<<sms * 8, threads, 0, st>>>(
+                launch_after(k_node_radius_listed<32>, sms * 8, threads, 0, st,
                     rlist + num_nodes - 1, -1, &bst->radius_mid, first, last, pos, stage, e.tris,
                     groups, r2bits);
             if (n > kRadiusChunk)
-                k_node_radius<<<sms * 8, 256, 0, st>>>(chunks, &bst->radius_chunks, max_chunks, last,
-                                                       pos, stage, e.tris, groups, r2bits);
+                launch_after(k_node_radius, sms * 8, 256, 0, st, chunks, &bst->radius_chunks,
+                    max_chunks, last, pos, stage, e.tris, groups, r2bits);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.records & FWN_RECORDS_F32)
@@ -3010,14 +3044,14 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         if (e.cfg.records & FWN_RECORDS_F64)
             e.nodes64 = static_cast<NodeF64*>(engine_alloc(E * sizeof(NodeF64), st));
         int* node_of_pos = arena.take<int>(E);
-        k_node_of_pos<<<grid_for(num_nodes, 256), 256, 0, st>>>(num_nodes, flags, pos, node_of_pos);
-        k_convert<<<grid_for(E, 128), 128, 0, st>>>(E, node_of_pos, keys, first, last, flags, skip,
-                                                    stage, r2bits, e.nodes32, e.nodes64,
-                                                    &bst->leaf_count);
+        launch_after(k_node_of_pos, grid_for(num_nodes, 256), 256, 0, st, num_nodes, flags, pos,
+            node_of_pos);
+        launch_after(k_convert, grid_for(E, 128), 128, 0, st, E, node_of_pos, keys, first, last,
+            flags, skip, stage, r2bits, e.nodes32, e.nodes64, &bst->leaf_count);
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.tuning == 7 && e.nodes32 && E > 0) {  // the structure-of-arrays layout variant
             e.soa = static_cast<float4*>(engine_alloc((size_t)E * sizeof(NodeF32), st));
-            k_aos_to_soa<<<grid_for(E, 256), 256, 0, st>>>(E, e.nodes32, e.soa);
+            launch_after(k_aos_to_soa, grid_for(E, 256), 256, 0, st, E, e.nodes32, e.soa);
             FWN_CUDA_CHECK(cudaGetLastError());
         }
     }

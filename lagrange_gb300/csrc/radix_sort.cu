@@ -68,6 +68,7 @@ __device__ __forceinline__ int block_exclusive_scan_256(int v, int* warp_tot) {
 template <class K>
 __global__ void __launch_bounds__(SORT_THREADS)
 k_upsweep(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hist, int nblocks) {
+    after_previous();
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ int wh[SORT_WARPS][RADIX];
     const int tid = threadIdx.x, w = tid >> 5;
@@ -92,6 +93,7 @@ k_upsweep(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hi
 // One block per digit: exclusive scan of that digit's per-tile counts (in place).
 __global__ void __launch_bounds__(1024)
 k_scan_digits(int* __restrict__ hist, int nblocks, int* __restrict__ digit_totals) {
+    after_previous();
     __shared__ int wt[32];
     __shared__ int carry_s;
     int* row = hist + (int64_t)blockIdx.x * nblocks;
@@ -135,6 +137,7 @@ constexpr int kFewTiles = 128;
 template <class K>
 __global__ void __launch_bounds__(SORT_THREADS)
 k_few_hist(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hist, int passes) {
+    after_previous();
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ int h[RADIX];
     const int tid = threadIdx.x;
@@ -165,6 +168,7 @@ k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
             K* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n, int shift,
             const int* __restrict__ hist, const int* __restrict__ digit_totals,
             int* __restrict__ hist_next, int nblocks) {
+    after_previous();
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ K skeys[TILE];
     __shared__ uint32_t svals[TILE];
@@ -294,20 +298,20 @@ bool radix_sort_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, int64_t n, int be
     bool in_b = false;
     const bool few = nblocks <= kFewTiles;
     if (few)
-        k_few_hist<K><<<nblocks, SORT_THREADS, 0, stream>>>(
-            ks, n, begin_bit, hist, (end_bit - begin_bit + RADIX_BITS - 1) / RADIX_BITS);
+        launch_after(k_few_hist<K>, nblocks, SORT_THREADS, 0, stream, ks, n, begin_bit, hist,
+            (end_bit - begin_bit + RADIX_BITS - 1) / RADIX_BITS);
     for (int shift = begin_bit; shift < end_bit; shift += RADIX_BITS) {
         if (few) {
             int* next = hist + (int64_t)RADIX * nblocks;
-            k_downsweep<K, true><<<nblocks, SORT_THREADS, 0, stream>>>(
-                ks, vs, kd, vd, n, shift, hist, nullptr, shift + RADIX_BITS < end_bit ? next : nullptr,
-                nblocks);
+            launch_after(k_downsweep<K, true>, nblocks, SORT_THREADS, 0, stream, ks, vs, kd, vd,
+                n, shift, hist, nullptr, shift + RADIX_BITS < end_bit ? next : nullptr, nblocks);
             hist = next;
         } else {
-            k_upsweep<K><<<nblocks, SORT_THREADS, 0, stream>>>(ks, n, shift, hist, nblocks);
-            k_scan_digits<<<RADIX, 1024, 0, stream>>>(hist, nblocks, totals);
-            k_downsweep<K, false><<<nblocks, SORT_THREADS, 0, stream>>>(ks, vs, kd, vd, n, shift, hist,
-                                                                        totals, nullptr, nblocks);
+            launch_after(k_upsweep<K>, nblocks, SORT_THREADS, 0, stream, ks, n, shift, hist,
+                nblocks);
+            launch_after(k_scan_digits, RADIX, 1024, 0, stream, hist, nblocks, totals);
+            launch_after(k_downsweep<K, false>, nblocks, SORT_THREADS, 0, stream, ks, vs, kd, vd,
+                n, shift, hist, totals, nullptr, nblocks);
         }
         std::swap(ks, kd);
         vs = vd;
@@ -365,6 +369,7 @@ __device__ __forceinline__ void load_items(const int* __restrict__ data, int64_t
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_tile_sums(const int* __restrict__ data, int64_t n, int* __restrict__ sums) {
+    after_previous();
     __shared__ int wt[32];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
     int v[SCAN_IPT];
@@ -380,6 +385,7 @@ k_scan_tile_sums(const int* __restrict__ data, int64_t n, int* __restrict__ sums
 // A few tiles by one block, one after the other: one launch of 2 to 6 us in place of three (12 us).
 constexpr int kScanFewTiles = 4;
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_few(int* __restrict__ data, int64_t n) {
+    after_previous();
     __shared__ int wt[32];
     int carry = 0;
     for (int64_t base = 0; base < n; base += SCAN_TILE) {
@@ -401,6 +407,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_few(int* __restrict__ dat
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* __restrict__ sums, int m) {
+    after_previous();
     __shared__ int wt[32];
     int carry = 0;
     for (int b = 0; b < m; b += SCAN_THREADS) {
@@ -415,6 +422,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* __restrict__ su
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_tiles(int* __restrict__ data, int64_t n, const int* __restrict__ sums) {
+    after_previous();
     __shared__ int wt[32];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
     const int64_t i0 = base + (int64_t)threadIdx.x * SCAN_IPT;
@@ -466,16 +474,16 @@ size_t exclusive_scan_temp_bytes(int64_t n) {
 
 void exclusive_scan_i32(int* data, int64_t n, void* temp, cudaStream_t stream) {
     if (n <= (int64_t)kScanFewTiles * SCAN_TILE) {
-        k_scan_few<<<1, SCAN_THREADS, 0, stream>>>(data, n);
+        launch_after(k_scan_few, 1, SCAN_THREADS, 0, stream, data, n);
         FWN_CUDA_CHECK(cudaGetLastError());
         return;
     }
     if (n <= 0) return;
     const int m = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     int* sums = static_cast<int*>(temp);
-    k_scan_tile_sums<<<m, SCAN_THREADS, 0, stream>>>(data, n, sums);
-    k_scan_sums<<<1, SCAN_THREADS, 0, stream>>>(sums, m);
-    k_scan_tiles<<<m, SCAN_THREADS, 0, stream>>>(data, n, sums);
+    launch_after(k_scan_tile_sums, m, SCAN_THREADS, 0, stream, data, n, sums);
+    launch_after(k_scan_sums, 1, SCAN_THREADS, 0, stream, sums, m);
+    launch_after(k_scan_tiles, m, SCAN_THREADS, 0, stream, data, n, sums);
     FWN_CUDA_CHECK(cudaGetLastError());
 }
 
