@@ -251,6 +251,16 @@ class Clocks:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
+def query_launches(n, max_queries, nodes, mesh_bits=0, key_bits=30):
+    """Kernels of one sorted query of n points (the library's choices): keys, the sort's passes, the
+    walk, the walk of left-over groups, the results' scatter and, from a million points, the
+    second output from the first."""
+    need = max(1, mesh_bits + math.ceil(math.log2(max_queries)) + (-1 if nodes <= 32768 else 2))
+    passes = min(math.ceil(need / 8), math.ceil(key_bits / 8))
+    sort = 1 + passes if n <= 128 * 2048 else 3 * passes
+    return 1 + sort + 2 + 1 + (1 if n >= 1_000_000 else 0)
+
+
 def measured_peaks():
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -730,8 +740,7 @@ def run_ours(args, rank, world, local):
         "step_ms_min": min(step_ms), "step_ms_median": statistics.median(step_ms),
         "wall_s_timed": t_wall,
         "split_queries_bit_identical": split_check,
-        # per step: keys + 4 sort passes x 3 kernels + traversal + result scatter
-        "gpu_launches": (1 + 4 * 3 + 1 + 1) * args.steps,
+        "gpu_launches": query_launches(n, n, info["num_nodes"]) * args.steps,
         "clocks": clocks,
     }
 
@@ -1125,7 +1134,8 @@ def measure_forest(fo, dev, dist, rank, world, *, leaf=0, builder=0, tuning=0, s
     ms = max_over_ranks(dist, sum(ts) / len(ts), dev)
     build_ms = min(builds)
     key_bits = fwn.forest_sort_key_bits(fo.qoff)  # the library's own choice for these offsets
-    launches_per_query = 1 + 3 * math.ceil(key_bits / 8) + 1 + 1  # keys, sort, walk, scatter
+    launches_per_query = query_launches(n, int(np.max(np.diff(fo.qoff))), forest.info()["num_nodes"] // M,
+                                        math.ceil(math.log2(M)), key_bits)
     result = {
         "metric": f"winding queries/s, {M} meshes in one persistent CUDA-graph launch",
         "value": job_value(n, world, ms / 1e3), "unit": "queries/s", "n_gpus": world,
