@@ -114,3 +114,24 @@ def test_radii_at_scales(torch, oracle_mod, builder, scale, shift):
     V, F = wl.V.astype(np.float64), wl.F.copy()
     F[::97, 1] = F[0, 0]
     _compare(oracle_mod, ((V + shift) * scale).astype(np.float32), F, 4, builder)
+
+
+@pytest.mark.parametrize("builder", [fwn.BUILDER_LBVH, fwn.BUILDER_SPLIT, fwn.BUILDER_BINNED])
+@pytest.mark.parametrize("fault", ["nan", "inf", "index", "negative"])
+def test_bad_input_of_a_large_mesh(torch, builder, fault):
+    """The levels that are launched before the input's check has come back run on whatever the bad
+    triangles gave; the build is refused, and the next one is right."""
+    wl = W.displaced_icosphere_workload(nu=60, n_queries=1)
+    V, F = wl.V.copy(), wl.F.copy()
+    if fault == "nan":
+        V[F[5000, 1]] = np.nan
+    elif fault == "inf":
+        V[F[123, 0]] = (np.inf, 0, -np.inf)
+    else:
+        F[7777, 2] = len(V) if fault == "index" else -1
+    good = fwn.FastWindingNumber(wl.V, wl.F, builder=builder).export_tree()
+    with pytest.raises(fwn.WindingError):
+        fwn.FastWindingNumber(V, F, builder=builder)
+    again = fwn.FastWindingNumber(wl.V, wl.F, builder=builder).export_tree()
+    for k in good:
+        np.testing.assert_array_equal(good[k], again[k])
