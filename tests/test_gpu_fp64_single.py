@@ -68,3 +68,13 @@ def test_special_points(torch, scale):
     bad = np.array([[np.nan, 0, 0], [np.inf, 0, 0], [0, -np.inf, 1]])
     eng = fwn.FastWindingNumber(V * scale, F, records=fwn.RECORDS_F64, beta=1e30)
     _compare(torch, eng, np.concatenate([Q, bad]))
+
+
+# queries of a few terms and of many, next to each other: batches that hold several queries' terms
+@pytest.mark.parametrize("n", [5, 4 * 152 * 128 + 3, 200_000])
+def test_mixed_neighbours(torch, n):
+    wl = W.displaced_icosphere_workload(nu=20, n_queries=n)
+    Q = wl.Q.copy()
+    Q[::3] = Q[::3] * 40 + 200  # far away: the root's term alone
+    Q[1::7] = wl.V[np.arange(len(Q[1::7])) % len(wl.V)]  # on vertices
+    _compare(torch, fwn.FastWindingNumber(wl.V, wl.F, records=fwn.RECORDS_F64, leaf_size=16), Q)
