@@ -38,3 +38,19 @@ def test_rounded_once(torch, nu, one_sum, tuning):
     for kw in ({}, {"traversal": fwn.TRAVERSAL_THREAD}):
         d = (eng.query(Q, **kw)[0].double() - w64) / FOUR_PI
         assert float(d.square().mean().sqrt()) <= 1.02 * one_sum
+
+
+# With a near distance beyond the mesh and cond = 0 every group's list runs full, so that the launch for
+# left-over groups answers; a warp per query gives the same bits
+@pytest.mark.parametrize("leaf", [8, 16])
+@pytest.mark.parametrize("tuning", [3, 6])
+def test_left_over_groups_have_the_same_bits(torch, tuning, leaf):
+    V, F = W.uv_sphere(16, 8)
+    box = W.box_queries(V, 300_000, np.random.default_rng(5))
+    Q = torch.from_numpy(np.concatenate([_near(V, F, 300_000, 4), box])).cuda()
+    cfg = {"fp64_cond": 0.0, "fp64_near_scale": 10.0, "leaf_size": leaf}
+    group = fwn.FastWindingNumber(V, F, tuning=tuning, **cfg)
+    one = fwn.FastWindingNumber(V, F, **cfg)
+    w = group.query(Q)[0]
+    alone = torch.cat([one.query(Q[i:i + 20_000])[0] for i in range(0, len(Q), 20_000)])
+    np.testing.assert_array_equal(w.cpu().numpy(), alone.cpu().numpy())
