@@ -44,6 +44,10 @@ cudaMemPool_t scratch_pool(int dev, int kind) {
             FWN_CUDA_CHECK(err);
         }
         g_pools[kind][dev] = pool;
+        // a small block that stays: beside it the engines' mesh tables take 2 us to allocate and free,
+        // 58 where each of them is the only block of its page
+        void* stays = nullptr;
+        if (kind == 2) FWN_CUDA_CHECK(cudaMalloc(&stays, 256));
     }
     return g_pools[kind][dev];
 }
@@ -96,21 +100,26 @@ void* engine_alloc(size_t bytes, cudaStream_t st) {
     return bytes ? pool_alloc(bytes, st, 2) : nullptr;
 }
 
+MeshInfo* mesh_table_alloc(int64_t count) {
+    void* p = nullptr;
+    FWN_CUDA_CHECK(cudaMalloc(&p, (size_t)count * sizeof(MeshInfo)));
+    return static_cast<MeshInfo*>(p);
+}
+
 Engine::~Engine() {
     // free on the engine's device, then give the caller back its current device
     int cur = -1;
     const bool swap = cudaGetDevice(&cur) == cudaSuccess && cur != device &&
                       cudaSetDevice(device) == cudaSuccess;
-    // work that still reads the engine may be in flight on any stream: wait for the device, as
-    // cudaFree does (which takes over where the device cannot be waited for)
-    void* own[] = {nodes32, nodes64, soa, tris, sorted_tri, meshes, stage};
-    bool waited = false, idle = false;
-    for (void* p : own) {
-        if (!p) continue;
-        if (!waited) idle = cudaDeviceSynchronize() == cudaSuccess;
-        waited = true;
-        if (!(idle && cudaFreeAsync(p, cudaStreamPerThread) == cudaSuccess)) cudaFree(p);
-    }
+    // Work that still reads the engine may be in flight on any stream, or in a graph. The mesh table is
+    // plain device memory, whose cudaFree waits for the device (cudaDeviceSynchronize would break
+    // captures of other threads that cudaFree leaves alone); freeing the pool's memory does not wait.
+    // Where cudaFree is refused (during some captures) the memory stays allocated.
+    void* own[] = {nodes32, nodes64, soa, tris, sorted_tri, stage};
+    bool ok = !meshes || cudaFree(meshes) == cudaSuccess;
+    for (void* p : own)
+        if (ok && p) ok = cudaFree(p) == cudaSuccess;
+    if (!ok) cudaGetLastError();  // a refusal is not the next call's error
     if (swap) cudaSetDevice(cur);
     delete[] meshes_h;
     delete[] node_tri_begin_h;

@@ -203,6 +203,7 @@ void* build_alloc(size_t bytes, cudaStream_t stream);
 // memory goes to the next one; the pool keeps at most kEngineRetainBytes that no engine uses.
 constexpr uint64_t kEngineRetainBytes = uint64_t(2) << 30;
 void* engine_alloc(size_t bytes, cudaStream_t stream);
+MeshInfo* mesh_table_alloc(int64_t count);  // plain device memory (see Engine::~Engine)
 
 struct Scratch {
     void* p = nullptr;

@@ -2669,7 +2669,7 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                                    cudaMemcpyHostToDevice, st));
     FWN_CUDA_CHECK(cudaMemcpyAsync(foff, foff_h, (nmeshes + 1) * sizeof(int64_t),
                                    cudaMemcpyHostToDevice, st));
-    e.meshes = static_cast<MeshInfo*>(engine_alloc(nmeshes * sizeof(MeshInfo), st));
+    e.meshes = mesh_table_alloc(nmeshes);
     e.meshes_h = new MeshInfo[nmeshes];
     unsigned* enc = arena.take<unsigned>(6 * nmeshes);
     BuildState* bst = arena.take<BuildState>(1);

@@ -231,7 +231,7 @@ extern "C" FWN_API fwn_status fwn_load(const char* path, fwn_handle* out) {
         e->nodes64 = to_device(n64);
         e->tris = to_device(tris);
         e->sorted_tri = to_device(sorted);
-        e->meshes = static_cast<MeshInfo*>(engine_alloc((size_t)M * sizeof(MeshInfo), 0));
+        e->meshes = mesh_table_alloc(M);
         FWN_CUDA_CHECK(cudaMemcpy(e->meshes, meshes.data(), (size_t)M * sizeof(MeshInfo),
                                   cudaMemcpyHostToDevice));
         e->meshes_h = new MeshInfo[(size_t)M];

@@ -1,0 +1,70 @@
+"""GPU tests of the engines' device memory: destroying an engine beside other work and captures."""
+import threading
+
+import numpy as np
+import pytest
+
+import lagrange_gb300 as fwn
+from lagrange_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    t = pytest.importorskip("torch")
+    if not t.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    return t
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_destroy_leaves_another_threads_capture_alone(torch, mode):
+    """A thread destroys an engine (and builds, queries and destroys another) while this one captures."""
+    V, F = W.uv_sphere(16, 8)
+    Q = np.random.default_rng(0).uniform(-1.5, 1.5, (5000, 3)).astype(np.float32)
+    doomed, kept = fwn.FastWindingNumber(V, F), fwn.FastWindingNumber(V, F)
+    want = kept.query(Q)[0]
+    x = torch.zeros(8, device="cuda")
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    got = []
+
+    def work():
+        doomed.close()
+        got.append(kept.query(Q)[0])
+        another = fwn.FastWindingNumber(V, F)
+        got.append(another.query(Q)[0])
+        another.close()
+
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        x += 1
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
+    assert len(got) == 2
+    for w in got:
+        np.testing.assert_array_equal(w, want)
+
+
+def test_destroy_waits_for_queries_in_flight(torch):
+    wl = W.displaced_icosphere_workload(nu=60, n_queries=1_000_000)
+    kept, doomed = fwn.FastWindingNumber(wl.V, wl.F), fwn.FastWindingNumber(wl.V, wl.F)
+    Q = torch.from_numpy(wl.Q).cuda()
+    want = kept.query(Q, traversal=fwn.TRAVERSAL_THREAD)[0]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        got = [doomed.query(Q, traversal=fwn.TRAVERSAL_THREAD)[0] for _ in range(4)]
+    doomed.close()
+    assert side.query()  # complete
+    other = W.displaced_icosphere_workload(nu=61, n_queries=1)
+    again = [fwn.FastWindingNumber(other.V, other.F) for _ in range(3)]  # into the same memory
+    torch.cuda.synchronize()
+    for w in got:
+        np.testing.assert_array_equal(w.cpu().numpy(), want.cpu().numpy())
+    del again
