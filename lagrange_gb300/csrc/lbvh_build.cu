@@ -2098,7 +2098,8 @@ constexpr int kGroup = 8;
 // What one warp looks at of the slots [s0, s1): t sees every vertex that can be the farthest from
 // P. A group's sphere (centre c, radius r about it, float) bounds its vertices: one lies at least
 // |c - P| away (c is their mean; rounding allowed for below), none farther than |c - P| + r.
-// known: a squared distance that some vertex of the node reaches (0: none known).
+// known: a squared distance that some vertex of the node reaches (0: none known; as large as m may
+// not be, it is not used: the cut's square would leave float's range and hide farther groups).
 // Vertices whose squared distance is 2e-5 below the largest cannot be it, in float or in double.
 __device__ __forceinline__ void screen_slots(const TriF32* __restrict__ tris,
                                              const float4* __restrict__ groups, int s0, int s1,
@@ -2116,7 +2117,7 @@ __device__ __forceinline__ void screen_slots(const TriF32* __restrict__ tris,
         if (m > 1e-30f && m < 1e36f) {  // squares neither underflow nor overflow
             const float d = sqrtf(m);
             least = d - 1e-6f * (3.f * d + fabsf(Pf[0]) + fabsf(Pf[1]) + fabsf(Pf[2]));
-            least = fmaxf(least, sqrtf(known) * 0.999999f);
+            if (known < 1e36f) least = fmaxf(least, sqrtf(known) * 0.999999f);
         }
     }
     if (!(least > 0.f)) {  // few groups, or no usable bound: every vertex
