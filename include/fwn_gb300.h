@@ -374,6 +374,13 @@ FWN_API fwn_status fwn_scratch_pool_stats(int32_t device, int32_t reset_high,
                                           uint64_t* reserved_bytes, uint64_t* used_bytes,
                                           uint64_t* used_high_bytes);
 
+/* No counterpart in the reference (its engine's memory is the host's). The library keeps freed device
+ * memory for its next calls: up to 8 GB of query scratch, 12 GB of build temporaries and 2 GB of
+ * destroyed engines per device. This call gives what nothing uses back to the driver, for other
+ * allocators on the device; memory of work still in flight stays (synchronise first to include
+ * it). */
+FWN_API fwn_status fwn_release_memory(int32_t device);
+
 /* No counterpart in the reference (its per-point queries sort nothing). The key width, in bits,
  * of the radix sort that fwn_forest_query runs for these HOST query offsets [num_meshes + 1]: the
  * mesh id above the top bits of the 30-bit Hilbert index, 32-bit keys while every mesh keeps at

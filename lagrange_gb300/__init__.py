@@ -90,7 +90,7 @@ EXPORTS = ["fwn_config_default", "fwn_last_error", "fwn_version", "fwn_build", "
            "fwn_forest_build_device", "fwn_forest_query", "fwn_query_noalloc", "fwn_autotune",
            "fwn_query_grid", "fwn_orientation_criterion", "fwn_query_order",
            "fwn_forest_autotune", "fwn_forest_sort_key_bits", "fwn_probe_fp32_peak",
-           "fwn_scratch_pool_stats", "fwn_save", "fwn_load"]
+           "fwn_scratch_pool_stats", "fwn_release_memory", "fwn_save", "fwn_load"]
 
 
 def library():
@@ -138,6 +138,7 @@ def library():
     L.fwn_probe_fp32_peak.argtypes = [C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double), P]
     u64p = C.POINTER(C.c_uint64)
     L.fwn_scratch_pool_stats.argtypes = [C.c_int32, C.c_int32, u64p, u64p, u64p]
+    L.fwn_release_memory.argtypes = [C.c_int32]
     L.fwn_save.argtypes = [P, C.c_char_p]
     L.fwn_load.argtypes = [C.c_char_p, C.POINTER(P)]
     for name in ("fwn_build", "fwn_build_device", "fwn_destroy", "fwn_get_info", "fwn_query",
@@ -147,7 +148,7 @@ def library():
                  "fwn_query_noalloc", "fwn_autotune", "fwn_query_grid",
                  "fwn_orientation_criterion", "fwn_query_order", "fwn_forest_autotune",
                  "fwn_forest_sort_key_bits", "fwn_probe_fp32_peak", "fwn_scratch_pool_stats",
-                 "fwn_save", "fwn_load"):
+                 "fwn_release_memory", "fwn_save", "fwn_load"):
         getattr(L, name).restype = st
     _lib = L
     return L
@@ -187,6 +188,12 @@ def scratch_pool_stats(device: int = 0, reset_high: bool = False) -> dict:
     _check(library().fwn_scratch_pool_stats(int(device), 1 if reset_high else 0, C.byref(r),
                                             C.byref(u), C.byref(h)))
     return {"reserved": r.value, "used": u.value, "used_high": h.value}
+
+
+def release_memory(device: int = 0) -> None:
+    """Gives the device memory that the library keeps for its next calls, and that nothing uses, back to
+    the driver (fwn_release_memory)."""
+    _check(library().fwn_release_memory(int(device)))
 
 
 def probe_fp32_peak(form: int = 0, stream=None) -> dict:

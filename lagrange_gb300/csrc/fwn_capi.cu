@@ -1,6 +1,7 @@
 // C ABI of the engine (declared in include/fwn_gb300.h). No exception crosses this boundary:
 // every entry point catches, stores the message in a thread-local slot and returns a status.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -25,7 +26,8 @@ std::mutex g_pool_mutex;
 // large build frees (in block sizes of its own) never stand in for a query's scratch and push the
 // query pool over its threshold
 cudaMemPool_t g_pools[3][kMaxDevices] = {};
-constexpr uint64_t kRetain[3] = {kScratchRetainBytes, kBuildRetainBytes, kEngineRetainBytes};
+constexpr uint64_t kRetain[3] = {kScratchRetainBytes, kBuildRetainBytes, UINT64_MAX};
+std::atomic<uint64_t> g_engine_bytes[kMaxDevices];  // of the live engines
 
 cudaMemPool_t scratch_pool(int dev, int kind) {
     if (dev < 0 || dev >= kMaxDevices) throw Error(FWN_INTERNAL, "device ordinal out of range");
@@ -96,8 +98,19 @@ void* scratch_alloc(size_t bytes, cudaStream_t st) { return pool_alloc(bytes, st
 
 void* build_alloc(size_t bytes, cudaStream_t st) { return pool_alloc(bytes, st, 1); }
 
-void* engine_alloc(size_t bytes, cudaStream_t st) {
-    return bytes ? pool_alloc(bytes, st, 2) : nullptr;
+void* engine_alloc(Engine& e, size_t bytes, cudaStream_t st) {
+    if (!bytes) return nullptr;
+    void* p = pool_alloc(bytes, st, 2);
+    e.pool_bytes += bytes;
+    g_engine_bytes[e.device] += bytes;
+    return p;
+}
+
+void release_memory(int dev) {
+    if (dev < 0 || dev >= kMaxDevices) throw Error(FWN_INVALID_ARG, "device ordinal out of range");
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (auto& kind : g_pools)
+        if (kind[dev]) FWN_CUDA_CHECK(cudaMemPoolTrimTo(kind[dev], 0));
 }
 
 MeshInfo* mesh_table_alloc(int64_t count) {
@@ -119,6 +132,15 @@ Engine::~Engine() {
     bool ok = !meshes || cudaFree(meshes) == cudaSuccess;
     for (void* p : own)
         if (ok && p) ok = cudaFree(p) == cudaSuccess;
+    if (ok && pool_bytes) {
+        const uint64_t live = g_engine_bytes[device] -= pool_bytes;
+        uint64_t held = 0;
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        const cudaMemPool_t pool = g_pools[2][device];
+        ok = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+             (held <= live + kEngineRetainBytes ||
+              cudaMemPoolTrimTo(pool, live + kEngineRetainBytes) == cudaSuccess);
+    }
     if (!ok) cudaGetLastError();  // a refusal is not the next call's error
     if (swap) cudaSetDevice(cur);
     delete[] meshes_h;
@@ -635,6 +657,10 @@ FWN_API fwn_status fwn_scratch_pool_stats(int32_t device, int32_t reset_high,
     return guarded([&] {
         scratch_pool_stats(device, reset_high != 0, reserved_bytes, used_bytes, used_high_bytes);
     });
+}
+
+FWN_API fwn_status fwn_release_memory(int32_t device) {
+    return guarded([&] { release_memory(device); });
 }
 
 FWN_API fwn_status fwn_forest_sort_key_bits(int64_t num_meshes, const int64_t* qoff,

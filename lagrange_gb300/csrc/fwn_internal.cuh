@@ -200,9 +200,13 @@ constexpr uint64_t kBuildRetainBytes = uint64_t(12) << 30;
 void* build_alloc(size_t bytes, cudaStream_t stream);
 // Engines live in a third pool: mapping and unmapping a 2-million-triangle engine's 190 MB with
 // cudaMalloc and cudaFree took 0.5 ms of a 3.8 ms build, query and destroy. A destroyed engine's
-// memory goes to the next one; the pool keeps at most kEngineRetainBytes that no engine uses.
+// memory goes to the next one, and the pool keeps at most kEngineRetainBytes that no engine uses:
+// the destructor trims it to that beside the live engines' bytes (a release threshold would count
+// those too, and keep nothing beside more than 2 GiB of engines).
 constexpr uint64_t kEngineRetainBytes = uint64_t(2) << 30;
-void* engine_alloc(size_t bytes, cudaStream_t stream);
+struct Engine;
+void* engine_alloc(Engine& e, size_t bytes, cudaStream_t stream);  // counted in e.pool_bytes
+void release_memory(int dev);  // what the pools of `dev` hold and nothing uses goes to the driver
 MeshInfo* mesh_table_alloc(int64_t count);  // plain device memory (see Engine::~Engine)
 
 struct Scratch {
@@ -252,6 +256,7 @@ struct Engine {
     TriF32* tris = nullptr;
     int* sorted_tri = nullptr;     // original triangle id per leaf slot
     MeshInfo* meshes = nullptr;    // device
+    uint64_t pool_bytes = 0;       // of the engine pool
     MeshInfo* meshes_h = nullptr;  // host copy
     StageRec* stage = nullptr;     // kept only when FWN_RECORDS_MOMENTS is requested
     int* node_tri_begin_h = nullptr;

@@ -2960,7 +2960,7 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         NvtxRange trace_refit("fwn build: FP64 refit, radii, records");
         StageRec* stage = nullptr;
         if (!(e.cfg.records & FWN_RECORDS_MOMENTS)) stage = arena.take<StageRec>(E);
-        else stage = e.stage = static_cast<StageRec*>(engine_alloc(E * sizeof(StageRec), st));
+        else stage = e.stage = static_cast<StageRec*>(engine_alloc(e, E * sizeof(StageRec), st));
         // the refit reads the records in 16 B pairs: the pool's allocations are 256 B aligned,
         // and a build that got less stops here rather than launch misaligned vector loads
         if (reinterpret_cast<uintptr_t>(stage) % alignof(StageRec) != 0)
@@ -3010,8 +3010,8 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
                     right, pos, stage, status);
         }
         FWN_CUDA_CHECK(cudaGetLastError());
-        e.tris = static_cast<TriF32*>(engine_alloc((size_t)n * sizeof(TriF32), st));
-        e.sorted_tri = static_cast<int*>(engine_alloc((size_t)n * sizeof(int), st));
+        e.tris = static_cast<TriF32*>(engine_alloc(e, (size_t)n * sizeof(TriF32), st));
+        e.sorted_tri = static_cast<int*>(engine_alloc(e, (size_t)n * sizeof(int), st));
         float4* groups = arena.take<float4>((n + kGroup - 1) / kGroup);
         launch_after(k_tri_records, grid_for(n, 256), 256, 0, st, n, tri_of_slot, keys, d_V, d_F,
             voff, e.tris, e.sorted_tri, groups);
@@ -3041,9 +3041,9 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
         }
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.records & FWN_RECORDS_F32)
-            e.nodes32 = static_cast<NodeF32*>(engine_alloc(E * sizeof(NodeF32), st));
+            e.nodes32 = static_cast<NodeF32*>(engine_alloc(e, E * sizeof(NodeF32), st));
         if (e.cfg.records & FWN_RECORDS_F64)
-            e.nodes64 = static_cast<NodeF64*>(engine_alloc(E * sizeof(NodeF64), st));
+            e.nodes64 = static_cast<NodeF64*>(engine_alloc(e, E * sizeof(NodeF64), st));
         int* node_of_pos = arena.take<int>(E);
         launch_after(k_node_of_pos, grid_for(num_nodes, 256), 256, 0, st, num_nodes, flags, pos,
             node_of_pos);
@@ -3051,7 +3051,7 @@ void build_forest(Engine& e, const float* d_V, const int64_t* voff_h, const int3
             flags, skip, stage, r2bits, e.nodes32, e.nodes64, &bst->leaf_count);
         FWN_CUDA_CHECK(cudaGetLastError());
         if (e.cfg.tuning == 7 && e.nodes32 && E > 0) {  // the structure-of-arrays layout variant
-            e.soa = static_cast<float4*>(engine_alloc((size_t)E * sizeof(NodeF32), st));
+            e.soa = static_cast<float4*>(engine_alloc(e, (size_t)E * sizeof(NodeF32), st));
             launch_after(k_aos_to_soa, grid_for(E, 256), 256, 0, st, E, e.nodes32, e.soa);
             FWN_CUDA_CHECK(cudaGetLastError());
         }

@@ -59,12 +59,10 @@ template <class T> std::vector<T> to_host(const T* d, int64_t n) {
     return h;
 }
 
-template <class T> T* to_device(const std::vector<T>& h) {
-    T* d = nullptr;
-    if (h.empty()) return nullptr;
-    d = static_cast<T*>(engine_alloc(h.size() * sizeof(T), 0));
+template <class T> void to_device(Engine& e, const std::vector<T>& h, T*& d) {
+    if (h.empty()) return;
+    d = static_cast<T*>(engine_alloc(e, h.size() * sizeof(T), 0));
     FWN_CUDA_CHECK(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return d;
 }
 
 void read_exact(FILE* f, void* p, size_t n, Fnv* sum) {
@@ -227,10 +225,10 @@ extern "C" FWN_API fwn_status fwn_load(const char* path, fwn_handle* out) {
         e->num_nodes = E;
         e->num_leaves = hd.num_leaves;
         e->leaf_cap = leaf_cap;
-        e->nodes32 = to_device(n32);
-        e->nodes64 = to_device(n64);
-        e->tris = to_device(tris);
-        e->sorted_tri = to_device(sorted);
+        to_device(*e, n32, e->nodes32);
+        to_device(*e, n64, e->nodes64);
+        to_device(*e, tris, e->tris);
+        to_device(*e, sorted, e->sorted_tri);
         e->meshes = mesh_table_alloc(M);
         FWN_CUDA_CHECK(cudaMemcpy(e->meshes, meshes.data(), (size_t)M * sizeof(MeshInfo),
                                   cudaMemcpyHostToDevice));

@@ -68,3 +68,34 @@ def test_destroy_waits_for_queries_in_flight(torch):
     for w in got:
         np.testing.assert_array_equal(w.cpu().numpy(), want.cpu().numpy())
     del again
+
+
+def test_memory_of_destroyed_engines(torch):
+    """Beside more than 2 GiB of live engines a destroyed one's memory stays for the next; of engines
+    destroyed together the library keeps 2 GiB at most, without a synchronisation; and that it gives
+    back when asked."""
+    MB = 1 << 20
+    every = fwn.RECORDS_F32 | fwn.RECORDS_F64 | fwn.RECORDS_MOMENTS
+    V, F = (torch.from_numpy(x).cuda() for x in W.displaced_icosphere(316, 1))
+    make = lambda: fwn.FastWindingNumber(V, F, records=every)  # noqa: E731
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    make().close()
+    torch.cuda.synchronize()
+    fwn.release_memory()
+    nothing = free()
+    live = [make() for _ in range(10)]
+    size = live[0].info()["device_bytes"]
+    assert 10 * size > 4 << 30
+    one = make()
+    torch.cuda.synchronize()
+    beside = free()
+    one.close()
+    torch.cuda.synchronize()
+    assert abs(free() - beside) < 64 * MB
+    for e in live:
+        e.close()
+    temporaries = 1 << 30  # of the builds, kept as well
+    assert nothing - free() < (2 << 30) + temporaries
+    torch.cuda.synchronize()
+    fwn.release_memory()
+    assert abs(free() - nothing) < 64 * MB
