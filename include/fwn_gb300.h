@@ -63,8 +63,8 @@ enum {
 };
 
 /* Traversal schedules. AUTO picks by form and batch: the mixed form's warp schedule, or for batches
- * too small to fill the GPU one warp per query (the same bits); one warp per query for the FP64
- * form. The FP64 form runs on the thread schedule (the plain form) or the warp schedule when THREAD
+ * too small to fill the GPU one warp per query (the same bits; an explicit WARP, or a tuning other
+ * than 0, keeps the warp schedule); one warp per query for the FP64 form. The FP64 form runs on the thread schedule (the plain form) or the warp schedule when THREAD
  * or WARP is asked for explicitly (FP64 arithmetic throughout; the schedules agree to 1e-12 in w). */
 enum {
     FWN_TRAVERSAL_AUTO = 0,   /* mixed: warp schedule; FP64 and small batches: a warp per query */

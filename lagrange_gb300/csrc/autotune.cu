@@ -150,6 +150,7 @@ extern "C" FWN_API fwn_status fwn_autotune(const float* d_V, int64_t nv, const i
                 QueryArgs a = resolve_query_args(e, nullptr);
                 a.precision = FWN_PRECISION_MIXED;
                 a.traversal = cand.traversal;
+                a.any_schedule = false;
                 a.block_size = cand.traversal == FWN_TRAVERSAL_WARP ? 128 : cand.block;
                 a.tuning = cand.tuning;
                 // one warm-up, then the median of three timed passes
@@ -249,6 +250,7 @@ extern "C" FWN_API fwn_status fwn_forest_autotune(const float* d_V, const int64_
             for (int tuning : {3, 1, 4, 5, 6}) {  // warp-schedule variants (queries per lane, cap)
                 QueryArgs a = resolve_query_args(e, nullptr);
                 a.precision = FWN_PRECISION_MIXED;
+                a.any_schedule = false;
                 a.tuning = tuning;
                 query_forest(e, a, d_Q, query_offsets, wbuf.as<float>(), ibuf.as<uint8_t>(), st);
                 float t[3];

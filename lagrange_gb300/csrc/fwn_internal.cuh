@@ -290,6 +290,7 @@ void build_forest(Engine& e, const float* d_vertices, const int64_t* vertex_offs
 struct QueryArgs {
     int precision = FWN_PRECISION_MIXED;
     int traversal = FWN_TRAVERSAL_THREAD;
+    bool any_schedule = false;  // the caller asked for none (AUTO)
     int block_size = 128;
     int sort_queries = 1;
     float beta = 2.0f;
