@@ -229,14 +229,17 @@ struct Scratch {
 // digits; the bits from end_bit up are zero. The values are the keys' places before the sort.
 // Sorts keys_a using keys_b as the other buffer; returns true when the keys and values ended in
 // the *_b buffers. temp holds 256 digit counts per tile of kSortTileKeys keys (for few tiles, of
-// every pass), plus the 256 digit totals (radix_sort_temp_bytes).
+// every pass), plus the 256 digit totals (radix_sort_temp_bytes). off (few tiles only, or null): a device
+// word that, where it is set, leaves everything as it is.
 // ---------------------------------------------------------------------------------------------
 constexpr int kSortTileKeys = 2048;  // keys per sort tile: 256 threads x 8 keys
 size_t radix_sort_temp_bytes(int64_t n, int key_bytes);
 bool radix_sort_u32(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b,
-                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream);
+                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream,
+                    const unsigned* off = nullptr);
 bool radix_sort_u64(uint64_t* keys_a, uint32_t* vals_a, uint64_t* keys_b, uint32_t* vals_b,
-                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream);
+                    int64_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream,
+                    const unsigned* off = nullptr);
 
 // Exclusive scan of n int32 values in place (radix_sort.cu).
 size_t exclusive_scan_temp_bytes(int64_t n);

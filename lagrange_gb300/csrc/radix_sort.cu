@@ -136,8 +136,10 @@ k_scan_digits(int* __restrict__ hist, int nblocks, int* __restrict__ digit_total
 constexpr int kFewTiles = 128;
 template <class K>
 __global__ void __launch_bounds__(SORT_THREADS)
-k_few_hist(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hist, int passes) {
+k_few_hist(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ hist, int passes,
+           const unsigned* __restrict__ off) {
     after_previous();
+    if (off && *off) return;
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ int h[RADIX];
     const int tid = threadIdx.x;
@@ -161,14 +163,15 @@ k_few_hist(const K* __restrict__ keys, int64_t n, int shift, int* __restrict__ h
 }
 
 // hist: of this pass, digit-major and scanned along the tiles; with FEW, the counts [tile][digit].
-// hist_next (FEW): the next pass's, or null.
+// hist_next (FEW): the next pass's, or null. off (FEW): nothing to do where it is set, or null.
 template <class K, bool FEW>
 __global__ void __launch_bounds__(SORT_THREADS)
 k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
             K* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n, int shift,
             const int* __restrict__ hist, const int* __restrict__ digit_totals,
-            int* __restrict__ hist_next, int nblocks) {
+            int* __restrict__ hist_next, int nblocks, const unsigned* __restrict__ off) {
     after_previous();
+    if (FEW && off && *off) return;
     constexpr int KPT = TileCfg<K>::KPT, TILE = TileCfg<K>::TILE;
     __shared__ K skeys[TILE];
     __shared__ uint32_t svals[TILE];
@@ -282,7 +285,7 @@ k_downsweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
 
 template <class K>
 bool radix_sort_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, int64_t n, int begin_bit,
-                     int end_bit, void* temp, cudaStream_t stream) {
+                     int end_bit, void* temp, cudaStream_t stream, const unsigned* off) {
     if (n <= 1 || end_bit <= begin_bit) {
         if (n == 1) FWN_CUDA_CHECK(cudaMemsetAsync(va, 0, sizeof(uint32_t), stream));
         return false;
@@ -297,21 +300,23 @@ bool radix_sort_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, int64_t n, int be
     uint32_t* vd = vb;
     bool in_b = false;
     const bool few = nblocks <= kFewTiles;
+    if (off && !few) throw Error(FWN_INTERNAL, "a sort of many tiles cannot be switched off");
     if (few)
         launch_after(k_few_hist<K>, nblocks, SORT_THREADS, 0, stream, ks, n, begin_bit, hist,
-            (end_bit - begin_bit + RADIX_BITS - 1) / RADIX_BITS);
+            (end_bit - begin_bit + RADIX_BITS - 1) / RADIX_BITS, off);
     for (int shift = begin_bit; shift < end_bit; shift += RADIX_BITS) {
         if (few) {
             int* next = hist + (int64_t)RADIX * nblocks;
             launch_after(k_downsweep<K, true>, nblocks, SORT_THREADS, 0, stream, ks, vs, kd, vd,
-                n, shift, hist, nullptr, shift + RADIX_BITS < end_bit ? next : nullptr, nblocks);
+                n, shift, hist, nullptr, shift + RADIX_BITS < end_bit ? next : nullptr, nblocks,
+                off);
             hist = next;
         } else {
             launch_after(k_upsweep<K>, nblocks, SORT_THREADS, 0, stream, ks, n, shift, hist,
                 nblocks);
             launch_after(k_scan_digits, RADIX, 1024, 0, stream, hist, nblocks, totals);
             launch_after(k_downsweep<K, false>, nblocks, SORT_THREADS, 0, stream, ks, vs, kd, vd,
-                n, shift, hist, totals, nullptr, nblocks);
+                n, shift, hist, totals, nullptr, nblocks, nullptr);
         }
         std::swap(ks, kd);
         vs = vd;
@@ -459,13 +464,13 @@ size_t radix_sort_temp_bytes(int64_t n, int key_bytes) {
 }
 
 bool radix_sort_u32(uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, int64_t n,
-                    int begin_bit, int end_bit, void* temp, cudaStream_t stream) {
-    return radix_sort_impl<uint32_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream);
+                    int begin_bit, int end_bit, void* temp, cudaStream_t stream, const unsigned* off) {
+    return radix_sort_impl<uint32_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream, off);
 }
 
 bool radix_sort_u64(uint64_t* ka, uint32_t* va, uint64_t* kb, uint32_t* vb, int64_t n,
-                    int begin_bit, int end_bit, void* temp, cudaStream_t stream) {
-    return radix_sort_impl<uint64_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream);
+                    int begin_bit, int end_bit, void* temp, cudaStream_t stream, const unsigned* off) {
+    return radix_sort_impl<uint64_t>(ka, va, kb, vb, n, begin_bit, end_bit, temp, stream, off);
 }
 
 size_t exclusive_scan_temp_bytes(int64_t n) {
