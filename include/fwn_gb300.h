@@ -112,7 +112,8 @@ typedef struct fwn_config {
                               records from a structure-of-arrays copy (eight float4 arrays,
                               128 B more per node) that a build with tuning 7 keeps: the layout
                               comparison, one mesh's point queries only (grids and forests run 6).
-                              0 (default): 6 for batches that fill the GPU, else 3 */
+                              0 (default): 6 for batches that fill the GPU (with fp64_cond at
+                              0.7 or above), else 3 */
     int32_t builder;       /* FWN_BUILDER_*. Default FWN_BUILDER_LBVH */
     int32_t reserved[5];
 } fwn_config;

@@ -54,3 +54,30 @@ def test_left_over_groups_have_the_same_bits(torch, tuning, leaf):
     w = group.query(Q)[0]
     alone = torch.cat([one.query(Q[i:i + 20_000])[0] for i in range(0, len(Q), 20_000)])
     np.testing.assert_array_equal(w.cpu().numpy(), alone.cpu().numpy())
+
+
+def _time(torch, f):
+    t = []
+    for _ in range(8):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        f()
+        b.record()
+        torch.cuda.synchronize()
+        t.append(a.elapsed_time(b))
+    return sorted(t[1:])[3]
+
+
+@pytest.mark.parametrize("n,cond", [(400_000, 0.0), (4_000_000, 0.5)])
+def test_low_conditions_walk_few_groups_twice(torch, n, cond):
+    """With a low fp64_cond most near triangles go to the lists. The thread walk has none, and no second
+    walk: the default took 1.44 and 1.32 times its time where groups whose lists ran full were walked
+    again by two blocks per SM, and two queries per lane whatever the condition."""
+    V, F = W.displaced_icosphere(224, 3)
+    eng = fwn.FastWindingNumber(V, F, fp64_cond=cond)
+    Q = torch.from_numpy(_near(V, F, n)).cuda()
+    w = eng.query(Q)[0]
+    t = eng.query(Q, traversal=fwn.TRAVERSAL_THREAD)[0]
+    assert float((w - t).abs().max()) / FOUR_PI <= 2e-6
+    thread = _time(torch, lambda: eng.query(Q, traversal=fwn.TRAVERSAL_THREAD))
+    assert _time(torch, lambda: eng.query(Q)) <= 1.2 * thread
