@@ -4,8 +4,10 @@
 // tuned at the caller's beta, which only changes how deep the walk goes).
 //
 // Optional cache: a text file with one line per (GPU name, log2 triangles, log2 queries) key:
-//   t2|<gpu name>|<log2 nf>|<log2 n> <leaf> <traversal> <block> <tuning> <builder> <ms>
-// A hit skips the timing; a miss appends the new line.
+//   t3|<gpu name>|<log2 nf>|<log2 n> <leaf> <traversal> <block> <tuning> <builder> <ms>
+// A hit skips the timing; a miss appends the new line. The first field changes with the kernels that the
+// choice was made for: t2 entries are of walks without lists of ill-conditioned triangles, whose best leaf
+// sizes are others.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -62,7 +64,7 @@ std::string cache_key(int64_t nf, int64_t n) {
     std::string name(prop.name);
     for (char& ch : name)
         if (ch == ' ' || ch == '|') ch = '_';
-    return "t2|" + name + "|" + std::to_string(log2_bucket(nf)) + "|" + std::to_string(log2_bucket(n));
+    return "t3|" + name + "|" + std::to_string(log2_bucket(nf)) + "|" + std::to_string(log2_bucket(n));
 }
 
 bool cache_lookup(const char* path, const std::string& key, fwn_tune_result* out) {
