@@ -275,9 +275,10 @@ FWN_API fwn_status fwn_export_moments(fwn_handle h, double* moments);
 FWN_API fwn_status fwn_export_nodes(fwn_handle h, void* nodes32, void* nodes64);
 
 /* Autotuner (no reference counterpart: the reference has no tunable parameters). For one mesh
- * (DEVICE arrays) and a representative DEVICE sample of query points, builds the tree with both
- * builders for leaf sizes 4, 8, 12 and 16 and times every query schedule (the warp cursor's variants 1-6; thread per
- * query with blocks of 64/128/256) with CUDA events; returns the fastest. Apply it
+ * (DEVICE arrays) and a representative DEVICE sample of query points, builds the tree with each
+ * builder for leaf sizes 4, 8, 12 and 16 and times every query schedule (the warp cursor's variants
+ * 1-6; thread per query with blocks of 64/128/256; for samples of 35,000 points or fewer AUTO with
+ * tuning 0 in place of variant 4) with CUDA events; returns the fastest. Apply it
  * with cfg.builder, cfg.leaf_size, cfg.traversal, cfg.block_size, cfg.tuning. `base` gives beta and the
  * precision knobs (NULL = defaults). cache_path (may be NULL) names a text file keyed by GPU name
  * and log2 of the triangle and query counts: a hit returns without timing, a miss appends.
@@ -291,8 +292,9 @@ FWN_API fwn_status fwn_autotune(const float* d_vertices, int64_t num_vertices,
  * so its knobs are the builder, the leaf size and the register cap: builds the forest (DEVICE
  * vertex/triangle arrays, HOST offset arrays as in fwn_forest_build_device) with both builders
  * for leaf sizes 4, 8, 12 and 16 and
- * times the forest query with tuning 3, 1, 4, 5 and 6 on the DEVICE points with HOST query_offsets
- * [num_meshes + 1]. Returns the fastest (builder, leaf size, tuning; traversal WARP, block 128). Cache as
+ * times the forest query with tuning 3, 1, 4, 5 and 6 (4 replaced as in fwn_autotune) on the DEVICE
+ * points with HOST query_offsets [num_meshes + 1]. Returns the fastest (builder, leaf size, tuning;
+ * traversal WARP, or AUTO for tuning 0; block 128). Cache as
  * in fwn_autotune, keyed also by log2 of the mesh count. Synchronous on `stream`. */
 FWN_API fwn_status fwn_forest_autotune(const float* d_vertices, const int64_t* vertex_offsets,
                                        const int32_t* d_triangles,

@@ -39,6 +39,10 @@ const Candidate kCandidates[] = {
     {FWN_TRAVERSAL_THREAD, 128, 0},
     {FWN_TRAVERSAL_THREAD, 256, 0},
 };
+// For a sample that AUTO answers with a warp per query on every tree, AUTO itself stands in place of
+// variant 4, which is 6 under another number: 4,096 queries of the UV sphere take 30 us with it, 195 with
+// the best named variant.
+constexpr int64_t kAutoSample = 35000;
 const int kLeafSizes[] = {4, 8, 12, 16};
 // One mesh (queried many times) tries all three builders; a forest, built for each batch, the two
 // whose build suits that (the binned splits add a binning pass per level for ~2% on the query).
@@ -151,10 +155,10 @@ extern "C" FWN_API fwn_status fwn_autotune(const float* d_V, int64_t nv, const i
             for (const Candidate& cand : kCandidates) {
                 QueryArgs a = resolve_query_args(e, nullptr);
                 a.precision = FWN_PRECISION_MIXED;
+                a.any_schedule = cand.tuning == 4 && n <= kAutoSample;
                 a.traversal = cand.traversal;
-                a.any_schedule = false;
                 a.block_size = cand.traversal == FWN_TRAVERSAL_WARP ? 128 : cand.block;
-                a.tuning = cand.tuning;
+                a.tuning = a.any_schedule ? 0 : cand.tuning;
                 // one warm-up, then the median of three timed passes
                 query_mesh(e, 0, a, d_Q, n, wbuf.as<float>(), ibuf.as<uint8_t>(), nullptr,
                            nullptr, st);
@@ -172,7 +176,7 @@ extern "C" FWN_API fwn_status fwn_autotune(const float* d_V, int64_t nv, const i
                 if (t[1] < best.ms) {
                     best.ms = t[1];
                     best.leaf_size = leaf;
-                    best.traversal = a.traversal;
+                    best.traversal = a.any_schedule ? FWN_TRAVERSAL_AUTO : a.traversal;
                     best.block_size = a.block_size;
                     best.tuning = a.tuning;
                     best.builder = builder;
@@ -252,8 +256,9 @@ extern "C" FWN_API fwn_status fwn_forest_autotune(const float* d_V, const int64_
             for (int tuning : {3, 1, 4, 5, 6}) {  // warp-schedule variants (queries per lane, cap)
                 QueryArgs a = resolve_query_args(e, nullptr);
                 a.precision = FWN_PRECISION_MIXED;
-                a.any_schedule = false;
-                a.tuning = tuning;
+                a.any_schedule = tuning == 4 && n <= kAutoSample;  // as for one mesh
+                a.traversal = FWN_TRAVERSAL_WARP;
+                a.tuning = a.any_schedule ? 0 : tuning;
                 query_forest(e, a, d_Q, query_offsets, wbuf.as<float>(), ibuf.as<uint8_t>(), st);
                 float t[3];
                 for (int r = 0; r < 3; ++r) {
@@ -268,9 +273,9 @@ extern "C" FWN_API fwn_status fwn_forest_autotune(const float* d_V, const int64_
                 if (t[1] < best.ms) {
                     best.ms = t[1];
                     best.leaf_size = leaf;
-                    best.traversal = FWN_TRAVERSAL_WARP;
+                    best.traversal = a.any_schedule ? FWN_TRAVERSAL_AUTO : FWN_TRAVERSAL_WARP;
                     best.block_size = 128;
-                    best.tuning = tuning;
+                    best.tuning = a.tuning;
                     best.builder = builder;
                 }
             }
