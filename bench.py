@@ -251,10 +251,13 @@ class Clocks:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
-def query_launches(n, max_queries, nodes, mesh_bits=0, key_bits=30):
+def query_launches(n, max_queries, nodes, mesh_bits=0, key_bits=30, auto=False):
     """Kernels of one sorted query of n points (the library's choices): keys, the sort's passes, the
     walk, the walk of left-over groups, the results' scatter and, from a million points, the
-    second output from the first."""
+    second output from the first. auto: the small batch of an engine whose schedule is AUTO, one
+    kernel."""
+    if auto and n <= 35_000:
+        return 1
     need = max(1, mesh_bits + math.ceil(math.log2(max_queries)) + (-1 if nodes <= 32768 else 2))
     passes = min(math.ceil(need / 8), math.ceil(key_bits / 8))
     sort = 1 + passes if n <= 128 * 2048 else 3 * passes
@@ -721,13 +724,13 @@ def run_ours(args, rank, world, local):
         "metric": METRIC, "value": value, "unit": "queries/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
         "scaling": "strong" if args.split_queries else "weak", "vs_baseline": None,
-        "dtype": "f32 (FP64 near field/refit)",
+        "dtype": "f32 (double-float/FP64 near field, FP64 refit)",
         "data": "synthetic",
         "config": {"workload": wl.name, "triangles": int(len(wl.F)),
                    "queries_per_gpu": n // world if args.split_queries else n,
                    "beta": wl.beta, "leaf_size": args.leaf,
                    "builder": BUILDER_NAMES.get(builder, str(builder)),
-                   "traversal": "warp" if trav == fwn.TRAVERSAL_WARP else "thread",
+                   "traversal": ("auto", "thread", "warp")[trav],
                    "block": args.block, "tuning": tuning, "autotuned": tuned,
                    "step": "plain launches" if args.no_graph else "CUDA graph of one query call",
                    "l2": "flushed before every step (256 MB write)",
@@ -740,7 +743,8 @@ def run_ours(args, rank, world, local):
         "step_ms_min": min(step_ms), "step_ms_median": statistics.median(step_ms),
         "wall_s_timed": t_wall,
         "split_queries_bit_identical": split_check,
-        "gpu_launches": query_launches(n, n, info["num_nodes"]) * args.steps,
+        "gpu_launches": query_launches(n, n, info["num_nodes"],
+                                       auto=trav == fwn.TRAVERSAL_AUTO and tuning == 0) * args.steps,
         "clocks": clocks,
     }
 
@@ -1135,12 +1139,12 @@ def measure_forest(fo, dev, dist, rank, world, *, leaf=0, builder=0, tuning=0, s
     build_ms = min(builds)
     key_bits = fwn.forest_sort_key_bits(fo.qoff)  # the library's own choice for these offsets
     launches_per_query = query_launches(n, int(np.max(np.diff(fo.qoff))), forest.info()["num_nodes"] // M,
-                                        math.ceil(math.log2(M)), key_bits)
+                                        math.ceil(math.log2(M)), key_bits, auto=tuning == 0)
     result = {
         "metric": f"winding queries/s, {M} meshes in one persistent CUDA-graph launch",
         "value": job_value(n, world, ms / 1e3), "unit": "queries/s", "n_gpus": world,
         "steps": steps, "warmup": warmup, "ms_per_step": ms, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f32 (FP64 near field/refit)",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f32 (double-float/FP64 near field, FP64 refit)",
         "data": "synthetic",
         "config": {"workload": fo.name, "meshes": M, "triangles": int(fo.foff[-1]),
                    "queries": n, "beta": fo.beta, "leaf_size": leaf,

@@ -64,8 +64,9 @@ enum {
 
 /* Traversal schedules. AUTO picks by form and batch: the mixed form's warp schedule, or for batches
  * too small to fill the GPU one warp per query (the same bits; an explicit WARP, or a tuning other
- * than 0, keeps the warp schedule); one warp per query for the FP64 form. The FP64 form runs on the thread schedule (the plain form) or the warp schedule when THREAD
- * or WARP is asked for explicitly (FP64 arithmetic throughout; the schedules agree to 1e-12 in w). */
+ * than 0, keeps the warp schedule); one warp per query for the FP64 form. The FP64 form runs on the
+ * thread schedule (the plain form) or the warp schedule when THREAD or WARP is asked for explicitly
+ * (FP64 arithmetic throughout; the schedules agree to 1e-12 in w). */
 enum {
     FWN_TRAVERSAL_AUTO = 0,   /* mixed: warp schedule; FP64 and small batches: a warp per query */
     FWN_TRAVERSAL_THREAD = 1, /* one thread per query, stackless skip-link walk */
@@ -129,12 +130,14 @@ typedef struct fwn_query_opts {
     int32_t reserved[6];
 } fwn_query_opts;
 
-/* Work counters of one query call (filled when a non-NULL pointer is passed to fwn_query_ex). */
+/* Work counters of one query call (filled when a non-NULL pointer is passed to fwn_query_ex): of the
+ * mixed form's group or thread walk, also for a small batch that AUTO would answer with a warp per
+ * query, and of the FP64 form's thread walk. */
 typedef struct fwn_query_stats {
     uint64_t nodes_tested;     /* node visits (far test evaluated) */
     uint64_t far_evals;        /* order-2 Taylor evaluations */
     uint64_t tri_evals;        /* exact triangle solid angles (all precisions) */
-    uint64_t tri_evals_fp64;   /* of which evaluated in FP64 (mixed form only) */
+    uint64_t tri_evals_fp64;   /* of which ill-conditioned: double-float or FP64 (mixed form only) */
     uint64_t warp_steps;       /* node steps summed over warps (max over the warp's lanes);
                                   the warp schedule counts with the variant's queries per lane
                                   (qpl = 2 for tunings >= 4): nodes_tested / (32 * qpl *

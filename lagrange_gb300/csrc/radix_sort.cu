@@ -478,12 +478,12 @@ size_t exclusive_scan_temp_bytes(int64_t n) {
 }
 
 void exclusive_scan_i32(int* data, int64_t n, void* temp, cudaStream_t stream) {
+    if (n <= 0) return;
     if (n <= (int64_t)kScanFewTiles * SCAN_TILE) {
         launch_after(k_scan_few, 1, SCAN_THREADS, 0, stream, data, n);
         FWN_CUDA_CHECK(cudaGetLastError());
         return;
     }
-    if (n <= 0) return;
     const int m = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     int* sums = static_cast<int*>(temp);
     launch_after(k_scan_tile_sums, m, SCAN_THREADS, 0, stream, data, n, sums);
