@@ -113,6 +113,16 @@ void release_memory(int dev) {
         if (kind[dev]) FWN_CUDA_CHECK(cudaMemPoolTrimTo(kind[dev], 0));
 }
 
+// cudaFreeHost, but as a call that this thread answers for: in the default mode it is refused while
+// another thread captures in the global mode, and breaks that capture.
+void free_pinned(void* p) {
+    if (!p) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaFreeHost(p);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 MeshInfo* mesh_table_alloc(int64_t count) {
     void* p = nullptr;
     FWN_CUDA_CHECK(cudaMalloc(&p, (size_t)count * sizeof(MeshInfo)));
@@ -217,8 +227,7 @@ HostStage* host_stage() {
     struct Stages {
         HostStage* s[kMaxDevices] = {};
         ~Stages() {
-            for (HostStage* x : s)
-                if (x) cudaFreeHost(x);
+            for (HostStage* x : s) free_pinned(x);
         }
     };
     thread_local Stages t;

@@ -206,6 +206,7 @@ void* build_alloc(size_t bytes, cudaStream_t stream);
 constexpr uint64_t kEngineRetainBytes = uint64_t(2) << 30;
 struct Engine;
 void* engine_alloc(Engine& e, size_t bytes, cudaStream_t stream);  // counted in e.pool_bytes
+void free_pinned(void* p);  // a thread's pinned memory when it ends, whatever other threads capture
 void release_memory(int dev);  // what the pools of `dev` hold and nothing uses goes to the driver
 MeshInfo* mesh_table_alloc(int64_t count);  // plain device memory (see Engine::~Engine)
 

@@ -2553,9 +2553,7 @@ public:
     StateReader(const BuildState* src, cudaStream_t s) : src_(src), s_(s) {
         struct Slots {
             Slot* p = nullptr;
-            ~Slots() {
-                if (p) cudaFreeHost(p);
-            }
+            ~Slots() { free_pinned(p); }
         };
         thread_local Slots t;
         if (!t.p) FWN_CUDA_CHECK(cudaHostAlloc(&t.p, 2 * sizeof(Slot), cudaHostAllocPortable));

@@ -1,5 +1,6 @@
 """GPU tests of the engines' device memory: destroying an engine beside other work and captures."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -99,3 +100,38 @@ def test_memory_of_destroyed_engines(torch):
     torch.cuda.synchronize()
     fwn.release_memory()
     assert abs(free() - nothing) < 64 * MB
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local"])
+@pytest.mark.parametrize("what", ["query", "build"])
+def test_thread_ends_beside_a_capture(torch, what, mode):
+    """A thread that queried host points, or built an engine, before a capture ends during it: the pinned
+    memory that it leaves is freed without breaking the capture."""
+    V, F = W.uv_sphere(16, 8)
+    eng = fwn.FastWindingNumber(V, F)
+    built = []
+    ready, go = threading.Event(), threading.Event()
+
+    def work():
+        if what == "query":
+            eng.query(np.zeros((3, 3), np.float32))
+        else:
+            built.append(fwn.FastWindingNumber(V, F))
+        ready.set()
+        go.wait()
+
+    t = threading.Thread(target=work)
+    t.start()
+    assert ready.wait(60)
+    x = torch.zeros(8, device="cuda")
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        x += 1
+        go.set()
+        t.join()
+        time.sleep(0.05)  # (the thread's own memory goes after its last Python statement)
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
