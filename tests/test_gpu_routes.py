@@ -150,3 +150,18 @@ def test_forests_around_the_lines(torch, meshes, kind):
     res = [fwn.Forest(Vs, off(len(V)), Fs, off(len(F)), tuning=t).query_forest(Q, off(each)) for t in (0, 3)]
     for a, b in zip(*res):
         np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
+
+
+@pytest.mark.parametrize("n,kw", [
+    (20_000, {"precision": fwn.PRECISION_FP64, "traversal": fwn.TRAVERSAL_WARP}),
+    (20_000, {"precision": fwn.PRECISION_FP64, "traversal": fwn.TRAVERSAL_THREAD}),
+    (100_000, {"beta": 3.0, "traversal": fwn.TRAVERSAL_WARP})])
+def test_sorted_walks_are_as_fast_as_ordered_ones(torch, n, kw):
+    """A walk after the sort takes the time of a walk over points that are in that order already, and the
+    sort's (60 us at most). Launches that overlapped the sort's end made it 1.13 to 1.22 times as long."""
+    V, F = W.displaced_icosphere(158, 3)
+    eng = fwn.FastWindingNumber(V, F, records=fwn.RECORDS_F32 | fwn.RECORDS_F64)
+    Q = torch.from_numpy(_batches(V, F, n)["mixed"]).cuda()
+    ordered = Q[eng.query_order(Q).long()].contiguous()
+    walk = _time(torch, lambda: eng.query(ordered, sort_queries=0, **kw))
+    assert _time(torch, lambda: eng.query(Q, **kw)) <= 1.06 * walk + 0.06
