@@ -35,7 +35,7 @@ def test_not_slower_than_the_default(torch):
     Q = torch.from_numpy(W.box_queries(V, 4096, np.random.default_rng(0))).cuda()
     r = fwn.autotune(V, F, Q)
     tuned, default = fwn.FastWindingNumber(V, F, **r["config"]), fwn.FastWindingNumber(V, F)
-    assert _time(torch, lambda: tuned.query(Q)) <= 1.5 * _time(torch, lambda: default.query(Q))
+    assert _time(torch, lambda: tuned.query(Q)) <= 2.0 * _time(torch, lambda: default.query(Q))
 
 
 def test_forest_not_slower_than_the_default(torch):
@@ -44,7 +44,7 @@ def test_forest_not_slower_than_the_default(torch):
     Q = torch.from_numpy(fo.Q).cuda()
     tuned, default = (fwn.Forest(fo.V, fo.voff, fo.F, fo.foff, **c) for c in (r["config"], {}))
     assert _time(torch, lambda: tuned.query_forest(Q, fo.qoff)) <= \
-        1.5 * _time(torch, lambda: default.query_forest(Q, fo.qoff))
+        2.0 * _time(torch, lambda: default.query_forest(Q, fo.qoff))
 
 
 def test_entries_of_other_kernels_are_not_used(torch, tmp_path):
